@@ -32,15 +32,17 @@ template <> struct Ar<float> {
 // multiply-add error-free product (Dekker 1971; Ogita, Rump and Oishi 2005);
 // rounding q + (f + e*x) once more gives the correctly rounded cube except
 // in rare ties, within the 1-ulp bound of the C library's pow.
-static __device__ __forceinline__ double cube(double x)
+// cube_p2 takes p = x*x rounded, where the caller has it.
+static __device__ __forceinline__ double cube_p2(double x, double p)
 {
-    double p = __dmul_rn(x, x);
     double e = __fma_rn(x, x, -p);
     double q = __dmul_rn(p, x);
     double f = __fma_rn(p, x, -q);
     return __dadd_rn(q, __fma_rn(e, x, f));
 }
+static __device__ __forceinline__ double cube(double x) { return cube_p2(x, __dmul_rn(x, x)); }
 static __device__ __forceinline__ float cube(float x) { return x * x * x; }
+static __device__ __forceinline__ float cube_p2(float x, float p) { return p * x; }
 
 // Model constants in the state type.
 template <typename T> struct P {
@@ -106,16 +108,23 @@ static __device__ __forceinline__ float noise_at(const P<float>& p, long long ce
     return gauss_at_f(p.seed, k) * (float)p.noise;
 }
 
-// 2.0*y, which is exact.  For FP64 a normal y whose double stays finite is
-// doubled by adding 1 to its exponent on the integer pipe; zeros,
-// subnormals, values near overflow, infinities and NaNs take the multiply.
-// Either way the bits are those of __dmul_rn(2.0, y).
+// 2.0*y, which is exact, on the integer pipe: a normal y whose double stays
+// finite has 1 added to its exponent.  Zeros and subnormals double by a shift
+// of the magnitude, the largest binade overflows to infinity, infinities and
+// NaNs stay: the value of __dmul_rn(2.0, y) in every case.  (A multiply for
+// the rare cases would be predicated, not branched over, and so cost an FP64
+// instruction per call: 25 instead of 23 per Cahn-Hilliard cell.)
 static __device__ __forceinline__ double twice(double y)
 {
-    const long long b = __double_as_longlong(y);
-    const unsigned e = (unsigned)((b >> 52) & 0x7ff);
-    if (e - 1u < 2045u) return __longlong_as_double(b + (1LL << 52));
-    return __dmul_rn(2.0, y);
+    const int hi = __double2hiint(y), lo = __double2loint(y);
+    const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+    if (e - 1u < 2045u) return __hiloint2double(hi + (1 << 20), lo);
+    const int sign = hi & (int)0x80000000;
+    if (e == 0u) {
+        const unsigned long long m = ((unsigned long long)(unsigned)(hi & 0x7fffffff) << 32 | (unsigned)lo) << 1;
+        return __longlong_as_double((long long)(m | (unsigned long long)(unsigned)sign << 32));
+    }
+    return e == 2046u ? __hiloint2double(sign | 0x7ff00000, 0) : y;
 }
 static __device__ __forceinline__ float twice(float y) { return 2.0f * y; }
 
