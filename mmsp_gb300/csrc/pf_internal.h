@@ -82,7 +82,7 @@ struct StepPlan {
     size_t smem;
     int planes;        // planes of axis X per block (3D streaming)
     int fields;
-    int kind;          // 0: generic tile kernel, 1: FP32 3D CH streaming, 2: FP32 3D AC streaming,
+    int kind;          // 0: the only kernel of its models' plan (CH tile, AC columns), 1: FP32 3D CH streaming,
                        // 3: FP32 CH rows of any length, 4: Ostwald ripening (two kernels),
                        // 5: convex splitting, 6: FP64 CH in two passes through a work grid,
                        // 8: FP32 3D Ostwald ripening streaming (one kernel)
@@ -112,12 +112,6 @@ bool ch_rows_eligible(const mmsp_gpu_desc& d, const Geom& g);
 cudaError_t plan_ch_rows(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 cudaError_t launch_ch_rows(const StepPlan& p, const mmsp_gpu_desc& d, const Coeffs& c, const void* in, void* out,
                            int* err, cudaStream_t s);
-
-// FP32 3D Allen-Cahn on whole rows (pf_ac3_stream.cu).
-bool ac3_stream_eligible(const mmsp_gpu_desc& d, const Geom& g);
-cudaError_t plan_ac3_stream(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
-cudaError_t launch_ac3_stream(const StepPlan& p, const Geom& g, const Coeffs& c, const void* in, void* out,
-                              int* err, cudaStream_t s);
 
 // A handle's device status block (256 bytes): int word 0 is set when a
 // kernel's bounded wait runs out, int word 1 when a sparse list overflows;
