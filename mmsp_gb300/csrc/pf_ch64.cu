@@ -20,8 +20,8 @@
 //
 // A thread owns one (y, z) column and walks a run of X planes, carrying
 // c(x-1), c(x), c(x+1) in registers; the four in-plane neighbours come
-// through L1 with periodic wraps precomputed per thread.  Blocks are small
-// (16 planes), so the block scheduler balances the FP64 work across SMs.
+// through L1 with periodic wraps precomputed per thread.  Blocks are small,
+// so the block scheduler balances the FP64 work across SMs.
 // Multiplies by 2 and the 0.0 + t of the Laplacian's first axis are done on
 // the integer pipe (pf_device.cuh), and every decision about parameters
 // (unit weights, kappa == 1, noise) is a template argument, so no FP64
@@ -33,7 +33,11 @@ namespace pf {
 
 constexpr int kC64Z = 32;        // block width along Z (one warp)
 constexpr int kC64Y = 4;         // rows per block: 128 threads
-constexpr int kC64Planes = 16;   // X planes per block (3D)
+// X planes per block (3D): short runs, so that small grids fill the SMs and
+// no SM is left with a long last block.  us per step at 16 / 2 planes, exact
+// form: 40^3 23.3 / 8.4, 100^3 72.3 / 59.7, 33x200x150 59.1 / 50.4, 256^3
+// 742 / 739 (a run of 1 measured as 2).
+constexpr int kC64Planes = 2;
 
 // Constants of both forms.
 struct C64 {
