@@ -213,24 +213,23 @@ ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcC
 // square p2 = phi*phi at hand.  KAPPA: 1 or 2 when kappa is exactly that
 // (1.0*x is x, 2.0*x is exact), 0 for any other value.
 template <typename T, int MODEL, int KAPPA, bool NOISE>
-static __device__ __forceinline__ T ac_new_p2(T phi, T p2, T sum, T lap, T noise, const P<T>& p)
+static __device__ __forceinline__ T ac_new_p2(const Ar<T>& A, T phi, T p2, T sum, T lap, T noise, const P<T>& p)
 {
-    using A = Ar<T>;
-    const T kl = KAPPA == 1 ? lap : KAPPA == 2 ? twice(lap) : A::mul(p.kappa, lap);
+    const T kl = KAPPA == 1 ? lap : KAPPA == 2 ? twice(lap) : A.mul(p.kappa, lap);
     if (MODEL == MMSP_GPU_AC) {
         // phi - dt*L*(-phi + phi*phi*phi + 2.0*gamma*phi*(sum - phi*phi) - kappa*lap)
-        const T a = A::add(-phi, A::mul(p2, phi));
-        const T g = A::mul(A::mul(p.gamma2, phi), A::sub(sum, p2));
-        return A::sub(phi, A::mul(p.dtm, A::sub(A::add(a, g), kl)));
+        const T a = A.add(-phi, A.mul(p2, phi));
+        const T g = A.mul(A.mul(p.gamma2, phi), A.sub(sum, p2));
+        return A.sub(phi, A.mul(p.dtm, A.sub(A.add(a, g), kl)));
     } else if (MODEL == MMSP_GPU_GG || MODEL == MMSP_GPU_ZENER) {
         // phi - dt*(-phi - pow(phi,3) + 2.0*(phi*sum - lap))   (graingrowth.cpp:105, zener.cpp:135)
-        const T e = A::add(A::sub(-phi, cube_p2(phi, p2)), twice(A::sub(A::mul(phi, sum), lap)));
-        return A::sub(phi, A::mul(p.dtm, e));
+        const T e = A.add(A.sub(-phi, cube_p2(A, phi, p2)), twice(A.sub(A.mul(phi, sum), lap)));
+        return A.sub(phi, A.mul(p.dtm, e));
     } else {
         // phi - dt*M*(-r*phi + u*pow(phi,3) - K*lap + noise)   (allen-cahn.cpp:70, model_A.cpp:99-100)
-        T e = A::sub(A::add(A::mul(p.neg_r, phi), A::mul(p.u, cube_p2(phi, p2))), kl);
-        if (NOISE) e = A::add(e, noise);
-        return A::sub(phi, A::mul(p.dtm, e));
+        T e = A.sub(A.add(A.mul(p.neg_r, phi), A.mul(p.u, cube_p2(A, phi, p2))), kl);
+        if (NOISE) e = A.add(e, noise);
+        return A.sub(phi, A.mul(p.dtm, e));
     }
 }
 
@@ -242,9 +241,10 @@ constexpr long long kAcAnySmall = 1LL << 17;
 
 template <typename T, int DIM, int MODEL, bool UNIT, int KAPPA, bool NOISE>
 __global__ void __launch_bounds__(kAcAnyThreads)
-ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> p, int N)
+ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> pc0, int N)
 {
-    using A = Ar<T>;
+    const Ar<T> A(g.dim);
+    const P<T> p = held(A, pc0);
     extern __shared__ __align__(8) unsigned char sq_raw[];
     T* mine = reinterpret_cast<T*>(sq_raw) + threadIdx.x;   // [field][thread]: this thread's squares
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,8 +263,8 @@ ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> p, int
 #pragma unroll 4
         for (int f = 0; f < N; f++) {
             const T c = __ldg(pc + f * g.cells);
-            const T p2 = A::mul(c, c);
-            sum = f == 0 ? p2 : A::add(sum, p2);
+            const T p2 = A.mul(c, c);
+            sum = f == 0 ? p2 : A.add(sum, p2);
             mine[f * blockDim.x] = p2;
         }
 #pragma unroll 2
@@ -274,8 +274,8 @@ ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> p, int
             T xl = T(0), xh = T(0), yl = T(0), yh = T(0);
             if (DIM == 3) xl = __ldg(q + dxl), xh = __ldg(q + dxh);
             if (DIM >= 2) yl = __ldg(q + dyl), yh = __ldg(q + dyh);
-            const T lap = lap_ref<T, UNIT, DIM>(twice(c), xh, xl, yh, yl, __ldg(q + dzh), __ldg(q + dzl), p.wx, p.wy, p.wz);
-            const T v = ac_new_p2<T, MODEL, KAPPA, NOISE>(c, mine[f * blockDim.x], sum, lap, noise, p);
+            const T lap = lap_ref<T, UNIT, DIM>(A, twice(c), xh, xl, yh, yl, __ldg(q + dzh), __ldg(q + dzl), p.wx, p.wy, p.wz);
+            const T v = ac_new_p2<T, MODEL, KAPPA, NOISE>(A, c, mine[f * blockDim.x], sum, lap, noise, p);
             // Zener pinning: the particles (field 0) have zero mobility (zener.cpp:134)
             po[f * g.cells] = (MODEL == MMSP_GPU_ZENER && f == 0) ? c : v;
         }

@@ -68,10 +68,9 @@ static __device__ __forceinline__ void st_row(T* __restrict__ dst, const T (&v)[
 // 2D Laplacian at cell j of a lane's row segment, reference order: axis 0
 // (rows) then axis 1 (cells of a row).
 template <typename T, int V, bool UNIT>
-static __device__ __forceinline__ T lap2(const T (&lo)[V], const T (&ce)[V], const T (&hi)[V], T left, T right,
+static __device__ __forceinline__ T lap2(const Ar<T>& A, const T (&lo)[V], const T (&ce)[V], const T (&hi)[V], T left, T right,
                                          int j, T w0, T w1)
 {
-    using A = Ar<T>;
     const T y = ce[j];
     const T zl = j == 0 ? left : ce[j - 1];
     const T zh = j == V - 1 ? right : ce[j + 1];
@@ -81,20 +80,20 @@ static __device__ __forceinline__ T lap2(const T (&lo)[V], const T (&ce)[V], con
         return fmaf(w0, hi[j] + lo[j], fmaf(w1, zh + zl, -2.0f * (w0 + w1) * y));
     } else {
         const T y2 = twice(y);
-        T lap = lap_axis<T, UNIT, true>(T(0), hi[j], y2, lo[j], w0);
-        return lap_axis<T, UNIT>(lap, zh, y2, zl, w1);
+        T lap = lap_axis<T, UNIT, true>(A, T(0), hi[j], y2, lo[j], w0);
+        return lap_axis<T, UNIT>(A, lap, zh, y2, zl, w1);
     }
 }
 
 // mu of the Cahn-Hilliard models; Horner's form in the precision form.
 template <typename T, int MODEL>
-static __device__ __forceinline__ T mu2(T c, T lap, const P<T>& p)
+static __device__ __forceinline__ T mu2(const Ar<T>& A, T c, T lap, const P<T>& p)
 {
     if constexpr (sizeof(T) == 4) {
         const float fp = MODEL == MMSP_GPU_CH ? c * fmaf(fmaf(4.0f, c, -6.0f), c, 2.0f) : c * fmaf(p.u, c * c, p.neg_r);
         return fmaf(-p.kappa, lap, fp);
     } else {
-        return ch_mu<T, MODEL>(c, lap, p);
+        return ch_mu<T, MODEL>(A, c, lap, p);
     }
 }
 
@@ -102,17 +101,17 @@ template <typename T, int V, int MODEL, bool UNIT>
 static __device__ void run_rows(const BatchInst& bi, int xs, int xe, const T* __restrict__ in, T* __restrict__ out,
                                 int lane)
 {
-    using A = Ar<T>;
     const int n0 = bi.n0, n1 = bi.n1;
+    const Ar<T> A(n1 >> 12);   // rows hold at most 512 cells
     const T* base_in = in + bi.off + lane * V;
     T* base_out = out + bi.off + lane * V;
     P<T> p;
-    p.kappa = (T)bi.kappa;
-    p.dtm = (T)bi.dtm;
-    p.neg_r = (T)bi.neg_r;
-    p.u = (T)bi.u;
+    p.kappa = A.reg((T)bi.kappa);
+    p.dtm = A.reg((T)bi.dtm);
+    p.neg_r = A.reg((T)bi.neg_r);
+    p.u = A.reg((T)bi.u);
     p.gamma2 = T(0);
-    const T w0 = (T)bi.w0, w1 = (T)bi.w1;
+    const T w0 = A.reg((T)bi.w0), w1 = A.reg((T)bi.w1);
     const unsigned FULL = 0xffffffffu;
     const int lm = (lane + 31) & 31, lp = (lane + 1) & 31;
 
@@ -135,13 +134,13 @@ static __device__ void run_rows(const BatchInst& bi, int xs, int xe, const T* __
         const T bl = __shfl_sync(FULL, c1[V - 1], lm);
         const T br = __shfl_sync(FULL, c1[0], lp);
 #pragma unroll
-        for (int j = 0; j < V; j++) m2[j] = mu2<T, MODEL>(c1[j], lap2<T, V, UNIT>(c0, c1, c2, bl, br, j, w0, w1), p);
+        for (int j = 0; j < V; j++) m2[j] = mu2<T, MODEL>(A, c1[j], lap2<T, V, UNIT>(A, c0, c1, c2, bl, br, j, w0, w1), p);
         if (x >= xs) {
             const T ml = __shfl_sync(FULL, m1[V - 1], lm);
             const T mr = __shfl_sync(FULL, m1[0], lp);
             T o[V];
 #pragma unroll
-            for (int j = 0; j < V; j++) o[j] = A::add(c0[j], A::mul(p.dtm, lap2<T, V, UNIT>(m0, m1, m2, ml, mr, j, w0, w1)));
+            for (int j = 0; j < V; j++) o[j] = A.add(c0[j], A.mul(p.dtm, lap2<T, V, UNIT>(A, m0, m1, m2, ml, mr, j, w0, w1)));
             st_row<T, V>(base_out + (long long)x * n1, o);
         }
 #pragma unroll

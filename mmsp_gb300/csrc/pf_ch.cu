@@ -38,9 +38,10 @@ struct ChTile {
 
 template <typename T, int DIM, int MODEL, int TY, bool UNIT_W>
 __global__ void __launch_bounds__(256)
-ch_step_kernel(const T* __restrict__ cin, T* __restrict__ cout, Geom g, P<T> p, int planes)
+ch_step_kernel(const T* __restrict__ cin, T* __restrict__ cout, Geom g, P<T> pc0, int planes)
 {
-    using A = Ar<T>;
+    const Ar<T> A(g.dim);
+    const P<T> p = held(A, pc0);
     using TL = ChTile<T, TY>;
     constexpr int CW = TL::CW, CH = TL::CH, CP = TL::CP, MW = TL::MW, MP = TL::MP;
     constexpr int NC = DIM == 3 ? 4 : 1, NM = DIM == 3 ? 3 : 1;
@@ -78,11 +79,11 @@ ch_step_kernel(const T* __restrict__ cin, T* __restrict__ cout, Geom g, P<T> p, 
             int ci = (my + 1) * CW + (mz + 1);
             T y = C[ci];
             T y2 = twice(y);
-            T lap = lap_ref<T, UNIT_W, DIM>(y2, H[ci], L[ci], C[ci + CW], C[ci - CW], C[ci + 1], C[ci - 1], p.wx,
+            T lap = lap_ref<T, UNIT_W, DIM>(A, y2, H[ci], L[ci], C[ci + CW], C[ci - CW], C[ci + 1], C[ci - 1], p.wx,
                                             p.wy, p.wz);
-            T mu = ch_mu<T, MODEL>(y, lap, p);
+            T mu = ch_mu<T, MODEL>(A, y, lap, p);
             // thermal noise of the stochastic forms (model_B.cpp:100-101, spinodal.cpp:95-97): mu + noise
-            if (p.noise != 0.0) mu = A::add(mu, noise_at(p, g.cells, pbase + yoff[my + 1] + zoff[mz + 1]));
+            if (p.noise != 0.0) mu = A.add(mu, noise_at(p, g.cells, pbase + yoff[my + 1] + zoff[mz + 1]));
             M[e] = mu;
         }
     };
@@ -100,10 +101,10 @@ ch_step_kernel(const T* __restrict__ cin, T* __restrict__ cout, Geom g, P<T> p, 
             int mi = (ly + 1) * MW + (lz + 1);
             T y = M[mi];
             T y2 = twice(y);
-            T lap = lap_ref<T, UNIT_W, DIM>(y2, MH[mi], ML[mi], M[mi + MW], M[mi - MW], M[mi + 1], M[mi - 1], p.wx,
+            T lap = lap_ref<T, UNIT_W, DIM>(A, y2, MH[mi], ML[mi], M[mi + MW], M[mi - MW], M[mi + 1], M[mi - 1], p.wx,
                                             p.wy, p.wz);
             T c = C[(ly + 2) * CW + (lz + 2)];
-            cout[(long long)gx * g.YZ + (long long)gy * g.Z + gz] = A::add(c, A::mul(p.dtm, lap));
+            cout[(long long)gx * g.YZ + (long long)gy * g.Z + gz] = A.add(c, A.mul(p.dtm, lap));
         }
     };
 

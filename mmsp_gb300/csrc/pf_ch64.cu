@@ -46,46 +46,66 @@ struct C64 {
     double w2;            // 2 (wx + wy + wz) over the real axes: the centre weight
     double poly0;         // contracted mu: 2 + kappa*w2 (CH) or -r + kappa*w2 (CH_POLY)
     double upd0;          // contracted update: -dt*M*w2
+    double four, six;     // contracted CH: set in the kernel
     double noise;
     unsigned long long seed;
     long long step;
 };
 
+// The constants of the expressions in registers (Ar::reg).
+static __device__ __forceinline__ C64 held(const Ar<double>& A, C64 q)
+{
+    q.wx = A.reg(q.wx);
+    q.wy = A.reg(q.wy);
+    q.wz = A.reg(q.wz);
+    q.kappa = A.reg(q.kappa);
+    q.dtm = A.reg(q.dtm);
+    q.u = A.reg(q.u);
+    q.poly0 = A.reg(q.poly0);
+    q.upd0 = A.reg(q.upd0);
+    q.four = A.reg(4.0);
+    q.six = A.reg(6.0);
+    return q;
+}
+
 // Weighted sum of the neighbour pairs (sx, sy, sz: sums of the two
 // neighbours along X, Y, Z), the contracted Laplacian without its centre term.
 template <int DIM, bool UNIT>
-static __device__ __forceinline__ double nsum(double sx, double sy, double sz, const C64& q)
+static __device__ __forceinline__ double nsum(const Ar<double>& A, double sx, double sy, double sz, const C64& q)
 {
-    if (UNIT) return DIM == 3 ? (sx + sy) + sz : sy + sz;
-    return DIM == 3 ? fma(q.wx, sx, fma(q.wy, sy, q.wz * sz)) : fma(q.wy, sy, q.wz * sz);
+    if (UNIT) return DIM == 3 ? A.add(A.add(sx, sy), sz) : A.add(sy, sz);
+    return DIM == 3 ? fma(q.wx, sx, fma(q.wy, sy, A.mul(q.wz, sz))) : fma(q.wy, sy, A.mul(q.wz, sz));
 }
 
 template <int DIM, int MODEL, bool UNIT, bool KONE, bool EXACT>
-static __device__ __forceinline__ double mu_cell(double c, double xh, double xl, double yh, double yl, double zh,
-                                                 double zl, const C64& q, const P<double>& p)
+static __device__ __forceinline__ double mu_cell(const Ar<double>& A, double c, double xh, double xl, double yh, double yl,
+                                                 double zh, double zl, const C64& q, const P<double>& p)
 {
     if (EXACT) {
         // temp = mu(c) in the reference's order (pf_device.cuh: lap_ref, ch_mu)
-        const double lap = lap_ref<double, UNIT, DIM>(twice(c), xh, xl, yh, yl, zh, zl, p.wx, p.wy, p.wz);
+        const double lap = lap_ref<double, UNIT, DIM>(A, twice(c), xh, xl, yh, yl, zh, zl, p.wx, p.wy, p.wz);
         P<double> pk = p;
         if (KONE) pk.kappa = 1.0;   // constant: kappa_times folds to lap
-        return ch_mu<double, MODEL>(c, lap, pk);
+        return ch_mu<double, MODEL>(A, c, lap, pk);
     }
     // mu = f'(c) - kappa (S - w2 c) = c * (poly0 + ...) - kappa S
-    const double s = nsum<DIM, UNIT>(xh + xl, yh + yl, zh + zl, q);
+    const double s = nsum<DIM, UNIT>(A, A.add(xh, xl), A.add(yh, yl), A.add(zh, zl), q);
     double t;
     if (MODEL == MMSP_GPU_CH) {   // 2c(1-c)(1-2c) = c (2 + c (-6 + 4c))
-        t = fma(fma(4.0, c, -6.0), c, q.poly0);
+        t = fma(fma(q.four, c, -q.six), c, q.poly0);
     } else {                      // -r c + u c^3 = c (-r + u c^2)
-        t = fma(q.u, c * c, q.poly0);
+        t = fma(q.u, A.mul(c, c), q.poly0);
     }
-    return KONE ? t * c - s : fma(-q.kappa, s, t * c);
+    return KONE ? fma(t, c, -s) : fma(-q.kappa, s, A.mul(t, c));
 }
 
 template <int DIM, int MODEL, bool UNIT, bool KONE, bool EXACT, bool NOISE>
 __global__ void __launch_bounds__(kC64Z * kC64Y)
-ch64_mu(const double* __restrict__ cin, double* __restrict__ mu, Geom g, C64 q, P<double> p, int planes)
+ch64_mu(const double* __restrict__ cin, double* __restrict__ mu, Geom g, C64 q0, P<double> p0, int planes)
 {
+    const Ar<double> A(g.dim);
+    const C64 q = held(A, q0);
+    const P<double> p = held(A, p0);
     const int z = blockIdx.x * kC64Z + threadIdx.x;
     const int y = blockIdx.y * kC64Y + threadIdx.y;
     if (z >= g.Z || y >= g.Y) return;   // no barrier in this kernel
@@ -104,10 +124,9 @@ ch64_mu(const double* __restrict__ cin, double* __restrict__ mu, Geom g, C64 q, 
         if (DIM == 3) n = __ldg(plane(x + 1 == g.X ? 0 : x + 1) + row + z);
         const double vyh = __ldg(pc + rh + z), vyl = __ldg(pc + rl + z);
         const double vzh = __ldg(pc + row + zh), vzl = __ldg(pc + row + zl);
-        double m = mu_cell<DIM, MODEL, UNIT, KONE, EXACT>(b, n, a, vyh, vyl, vzh, vzl, q, p);
+        double m = mu_cell<DIM, MODEL, UNIT, KONE, EXACT>(A, b, n, a, vyh, vyl, vzh, vzl, q, p);
         // thermal noise of the stochastic forms (model_B.cpp:100-101, spinodal.cpp:95-97): mu + noise
-        if (NOISE) m = EXACT ? __dadd_rn(m, noise_at(p, g.cells, (long long)x * g.YZ + row + z))
-                             : m + noise_at(p, g.cells, (long long)x * g.YZ + row + z);
+        if (NOISE) m = A.add(m, noise_at(p, g.cells, (long long)x * g.YZ + row + z));
         mu[(long long)x * g.YZ + row + z] = m;
         a = b;
         b = n;
@@ -116,9 +135,12 @@ ch64_mu(const double* __restrict__ cin, double* __restrict__ mu, Geom g, C64 q, 
 
 template <int DIM, bool UNIT, bool EXACT>
 __global__ void __launch_bounds__(kC64Z * kC64Y)
-ch64_update(const double* __restrict__ cin, const double* __restrict__ mu, double* __restrict__ cout, Geom g, C64 q,
-            P<double> p, int planes)
+ch64_update(const double* __restrict__ cin, const double* __restrict__ mu, double* __restrict__ cout, Geom g, C64 q0,
+            P<double> p0, int planes)
 {
+    const Ar<double> A(g.dim);
+    const C64 q = held(A, q0);
+    const P<double> p = held(A, p0);
     const int z = blockIdx.x * kC64Z + threadIdx.x;
     const int y = blockIdx.y * kC64Y + threadIdx.y;
     if (z >= g.Z || y >= g.Y) return;
@@ -142,11 +164,11 @@ ch64_update(const double* __restrict__ cin, const double* __restrict__ mu, doubl
         double o;
         if (EXACT) {
             // newGrid(n) = GRID(n) + dt*M*lap(temp)   (cahn-hilliard.cpp:75-76)
-            const double lap = lap_ref<double, UNIT, DIM>(twice(b), n, a, myh, myl, mzh, mzl, p.wx, p.wy, p.wz);
-            o = __dadd_rn(c, __dmul_rn(p.dtm, lap));
+            const double lap = lap_ref<double, UNIT, DIM>(A, twice(b), n, a, myh, myl, mzh, mzl, p.wx, p.wy, p.wz);
+            o = A.add(c, A.mul(p.dtm, lap));
         } else {
             // c + dtM (S - w2 mu) = fma(dtM, S, c - dtM w2 mu)
-            const double s = nsum<DIM, UNIT>(n + a, myh + myl, mzh + mzl, q);
+            const double s = nsum<DIM, UNIT>(A, A.add(n, a), A.add(myh, myl), A.add(mzh, mzl), q);
             o = fma(q.dtm, s, fma(q.upd0, b, c));
         }
         cout[i] = o;

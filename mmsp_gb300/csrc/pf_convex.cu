@@ -22,6 +22,15 @@ struct CsArgs {
     double wx, wy, wz;   // 1/dx^2 of padded axes X, Y, Z
 };
 
+// The constants of the expressions in registers (Ar::reg).
+static __device__ __forceinline__ CsArgs held(const Ar<double>& A, CsArgs a)
+{
+    double* v = &a.q.A12;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(CsArgs) / sizeof(double)); i++) v[i] = A.reg(v[i]);
+    return a;
+}
+
 struct CsNb {
     long long xh, xl, yh, yl;
     int zh, zl;
@@ -41,40 +50,39 @@ static __device__ __forceinline__ CsNb cs_row(const Geom& g, int x, int y)
 // fringe_laplacian (cahn-hilliard.cpp:155-170): sum over axes of
 // weight * (yh + yl), the Laplacian without its central term.
 template <int DIM>
-static __device__ __forceinline__ double fringe(const double* __restrict__ f, long long i, const CsNb& n,
-                                                const CsArgs& a)
+static __device__ __forceinline__ double fringe(const Ar<double>& A, const double* __restrict__ f, long long i,
+                                                const CsNb& n, const CsArgs& a)
 {
-    using A = Ar<double>;
     double s = 0.0;
-    if (DIM == 3) s = plus_zero(A::mul(a.wx, A::add(f[i + n.xh], f[i + n.xl])));
-    if (DIM == 3) s = A::add(s, A::mul(a.wy, A::add(f[i + n.yh], f[i + n.yl])));
-    if (DIM == 2) s = plus_zero(A::mul(a.wy, A::add(f[i + n.yh], f[i + n.yl])));
-    const double tz = A::mul(a.wz, A::add(f[i + n.zh], f[i + n.zl]));
-    return DIM == 1 ? plus_zero(tz) : A::add(s, tz);
+    if (DIM == 3) s = plus_zero(A.mul(a.wx, A.add(f[i + n.xh], f[i + n.xl])));
+    if (DIM == 3) s = A.add(s, A.mul(a.wy, A.add(f[i + n.yh], f[i + n.yl])));
+    if (DIM == 2) s = plus_zero(A.mul(a.wy, A.add(f[i + n.yh], f[i + n.yl])));
+    const double tz = A.mul(a.wz, A.add(f[i + n.zh], f[i + n.zl]));
+    return DIM == 1 ? plus_zero(tz) : A.add(s, tz);
 }
 
 template <int DIM>
-static __device__ __forceinline__ double field_lap(const double* __restrict__ f, long long i, const CsNb& n,
+static __device__ __forceinline__ double field_lap(const Ar<double>& A, const double* __restrict__ f, long long i, const CsNb& n,
                                                    const CsArgs& a)
 {
-    return lap_ref<double, false, DIM>(twice(f[i]), f[i + n.xh], f[i + n.xl], f[i + n.yh], f[i + n.yl], f[i + n.zh],
+    return lap_ref<double, false, DIM>(A, twice(f[i]), f[i + n.xh], f[i + n.xl], f[i + n.yh], f[i + n.yl], f[i + n.zh],
                                        f[i + n.zl], a.wx, a.wy, a.wz);
 }
 
 // expansive_dfdc (cahn-hilliard.cpp:92-96): -A*(C-C0) - QB*pow(C,2.0) - QD
-static __device__ __forceinline__ double expansive(double C, const CsConst& q)
+static __device__ __forceinline__ double expansive(const Ar<double>& A, double C, const CsConst& q)
 {
-    using A = Ar<double>;
-    return A::sub(A::sub(A::mul(-q.A, A::sub(C, q.C0)), A::mul(q.QB, A::mul(C, C))), q.QD);
+    return A.sub(A.sub(A.mul(-q.A, A.sub(C, q.C0)), A.mul(q.QB, A.mul(C, C))), q.QD);
 }
 
 // One color of the red-black sweep (cahn-hilliard.cpp:325-345): cells whose
 // coordinate sum has the parity `skip` are left alone, as `continue` does.
 template <int DIM>
 __global__ void __launch_bounds__(256)
-cs_sweep(const double* __restrict__ old, double* __restrict__ nw, Geom g, CsArgs a, int skip)
+cs_sweep(const double* __restrict__ old, double* __restrict__ nw, Geom g, CsArgs a0, int skip)
 {
-    using A = Ar<double>;
+    const Ar<double> A(g.dim);
+    const CsArgs a = held(A, a0);
     const CsConst& q = a.q;
     const long long rows = (long long)g.X * g.Y;
     const double* c1 = nw;              // guess, field 0
@@ -89,15 +97,15 @@ cs_sweep(const double* __restrict__ old, double* __restrict__ nw, Geom g, CsArgs
             const long long i = row * g.Z + z;
             const double cOld = old[i];
             const double cGuess = c1[i], uGuess = u1[i];
-            const double nonlin = A::add(A::mul(q.QA, A::mul(cGuess, cGuess)), q.QC);   // nonlinear_coeff
-            const double A21 = A::sub(-nonlin, q.KL);
-            const double detA = A::sub(1.0, A::mul(q.A12, A21));
-            const double B1 = A::add(cOld, A::mul(q.Ddt, fringe<DIM>(u1, i, n, a)));
-            const double B2 = A::sub(expansive(cOld, q), A::mul(q.K, fringe<DIM>(c1, i, n, a)));
-            const double cNew = __ddiv_rn(A::sub(B1, A::mul(B2, q.A12)), detA);
-            const double uNew = __ddiv_rn(A::sub(B2, A::mul(B1, A21)), detA);
-            nw[i] = A::add(A::mul(q.omega, cNew), A::mul(q.om1, cGuess));
-            nw[g.cells + i] = A::add(A::mul(q.omega, uNew), A::mul(q.om1, uGuess));
+            const double nonlin = A.add(A.mul(q.QA, A.mul(cGuess, cGuess)), q.QC);   // nonlinear_coeff
+            const double A21 = A.sub(-nonlin, q.KL);
+            const double detA = A.sub(A.one, A.mul(q.A12, A21));
+            const double B1 = A.add(cOld, A.mul(q.Ddt, fringe<DIM>(A, u1, i, n, a)));
+            const double B2 = A.sub(expansive(A, cOld, q), A.mul(q.K, fringe<DIM>(A, c1, i, n, a)));
+            const double cNew = __ddiv_rn(A.sub(B1, A.mul(B2, q.A12)), detA);
+            const double uNew = __ddiv_rn(A.sub(B2, A.mul(B1, A21)), detA);
+            nw[i] = A.add(A.mul(q.omega, cNew), A.mul(q.om1, cGuess));
+            nw[g.cells + i] = A.add(A.mul(q.omega, uNew), A.mul(q.om1, uGuess));
         }
     }
 }
@@ -115,14 +123,15 @@ static __device__ __forceinline__ void cs_add(CsNS& a, double x)
 }
 
 // Residual of the original system (cahn-hilliard.cpp:353-380): per cell
-// R1 = cOld - (cNew - D*dt*lap u), R2 = expansive(cOld) - (uNew -
+// R1 = cOld - (cNew - D*dt*lap u), R2 = expansive(A, cOld) - (uNew -
 // contractive(cNew) + K*lap c); sums of R1^2 + R2^2 and of B1^2 + B2^2.
 template <int DIM>
 __global__ void __launch_bounds__(256)
-cs_residual(const double* __restrict__ old, const double* __restrict__ nw, Geom g, CsArgs a,
+cs_residual(const double* __restrict__ old, const double* __restrict__ nw, Geom g, CsArgs a0,
             double* __restrict__ partials)
 {
-    using A = Ar<double>;
+    const Ar<double> A(g.dim);
+    const CsArgs a = held(A, a0);
     const CsConst& q = a.q;
     CsNS r{0.0, 0.0}, b{0.0, 0.0};
     const long long rows = (long long)g.X * g.Y;
@@ -135,17 +144,17 @@ cs_residual(const double* __restrict__ old, const double* __restrict__ nw, Geom 
             n.zh = z + 1 == g.Z ? -z : 1;
             n.zl = z == 0 ? g.Z - 1 : -1;
             const long long i = row * g.Z + z;
-            const double lapC = field_lap<DIM>(c1, i, n, a);
-            const double lapU = field_lap<DIM>(u1, i, n, a);
+            const double lapC = field_lap<DIM>(A, c1, i, n, a);
+            const double lapU = field_lap<DIM>(A, u1, i, n, a);
             const double cOld = old[i], cNew = c1[i], uNew = u1[i];
             const double B1 = cOld;
-            const double B2 = expansive(cOld, q);
-            const double AX1 = A::sub(cNew, A::mul(q.Ddt, lapU));
-            const double contr = A::add(A::mul(q.QA, cube(cNew)), A::mul(q.QC, cNew));   // contractive_dfdc
-            const double AX2 = A::add(A::sub(uNew, contr), A::mul(q.K, lapC));
-            const double R1 = A::sub(B1, AX1), R2 = A::sub(B2, AX2);
-            cs_add(r, A::add(A::mul(R1, R1), A::mul(R2, R2)));
-            cs_add(b, A::add(A::mul(B1, B1), A::mul(B2, B2)));
+            const double B2 = expansive(A, cOld, q);
+            const double AX1 = A.sub(cNew, A.mul(q.Ddt, lapU));
+            const double contr = A.add(A.mul(q.QA, cube(A, cNew)), A.mul(q.QC, cNew));   // contractive_dfdc
+            const double AX2 = A.add(A.sub(uNew, contr), A.mul(q.K, lapC));
+            const double R1 = A.sub(B1, AX1), R2 = A.sub(B2, AX2);
+            cs_add(r, A.add(A.mul(R1, R1), A.mul(R2, R2)));
+            cs_add(b, A.add(A.mul(B1, B1), A.mul(B2, B2)));
         }
     }
     // block: warp shuffles, then one thread per block in warp order

@@ -10,21 +10,49 @@
 namespace pf {
 
 // Arithmetic of the two forms.  The FP64 (plain) form rounds every operation
-// separately with the _rn intrinsics, so nothing is fused into a
-// multiply-add: that is how the reference's serial x86-64 build evaluates
-// the same expressions, and it keeps the device result bit-identical to it.
-// The FP32 (precision) form uses ordinary operators and lets the compiler
+// separately: that is how the reference's serial x86-64 build evaluates the
+// same expressions, and it keeps the device result bit-identical to it.  The
+// FP32 (precision) form uses ordinary operators and lets the compiler
 // contract them.
+//
+// On sm_103a the FP64 pipe takes a fused multiply-add of three vector
+// registers every 16 cycles per SM and warp, but an add, a multiply or a
+// multiply-add with a constant operand only every 19 (0.60 against 0.51 T
+// operations per second, 8 chains per thread, all SMs full).  So an add is
+// issued as a*1 + b and a multiply as a*b + (-0): rounded once, they have the
+// bits of the add and of the multiply, signed zeros included.  The 1 and the
+// -0 must be registers that the compiler cannot take for constants: they are
+// built from a value that is zero but only known at run time.  Constants of a
+// kernel's expressions go through reg() for the same reason.  us per step
+// with add, multiply and constant operands / in this form: Cahn-Hilliard 256^3
+// 739 / 628 (contracted 479 / 411), Allen-Cahn 128^3 x 8 608 / 515, Ostwald
+// 256x128x64 x 2 347 / 291.
 template <typename T> struct Ar;
 template <> struct Ar<double> {
-    static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
-    static __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    double one, mz;
+    int k;   // zero
+    // small: a value of at most 3 that the compiler does not know (a grid's dim)
+    explicit __device__ __forceinline__ Ar(int small)
+    {
+        k = (int)(threadIdx.x & ((unsigned)small >> 2));
+        one = __hiloint2double(0x3ff00000 | k, k);
+        mz = __hiloint2double((int)0x80000000 | k, k);
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, mz); }
+    __device__ __forceinline__ double reg(double a) const
+    {
+        return __hiloint2double(__double2hiint(a) | k, __double2loint(a) | k);   // on the integer pipe
+    }
 };
 template <> struct Ar<float> {
-    static __device__ __forceinline__ float add(float a, float b) { return a + b; }
-    static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
-    static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
+    static constexpr float one = 1.0f;
+    explicit __device__ __forceinline__ Ar(int) {}
+    __device__ __forceinline__ float add(float a, float b) const { return a + b; }
+    __device__ __forceinline__ float sub(float a, float b) const { return a - b; }
+    __device__ __forceinline__ float mul(float a, float b) const { return a * b; }
+    __device__ __forceinline__ float reg(float a) const { return a; }
 };
 
 // x^3 for the shipped examples' pow(x,3).  The exact cube is
@@ -33,16 +61,16 @@ template <> struct Ar<float> {
 // rounding q + (f + e*x) once more gives the correctly rounded cube except
 // in rare ties, within the 1-ulp bound of the C library's pow.
 // cube_p2 takes p = x*x rounded, where the caller has it.
-static __device__ __forceinline__ double cube_p2(double x, double p)
+static __device__ __forceinline__ double cube_p2(const Ar<double>& A, double x, double p)
 {
     double e = __fma_rn(x, x, -p);
-    double q = __dmul_rn(p, x);
+    double q = A.mul(p, x);
     double f = __fma_rn(p, x, -q);
-    return __dadd_rn(q, __fma_rn(e, x, f));
+    return A.add(q, __fma_rn(e, x, f));
 }
-static __device__ __forceinline__ double cube(double x) { return cube_p2(x, __dmul_rn(x, x)); }
-static __device__ __forceinline__ float cube(float x) { return x * x * x; }
-static __device__ __forceinline__ float cube_p2(float x, float p) { return p * x; }
+static __device__ __forceinline__ double cube(const Ar<double>& A, double x) { return cube_p2(A, x, A.mul(x, x)); }
+static __device__ __forceinline__ float cube_p2(const Ar<float>&, float x, float p) { return p * x; }
+static __device__ __forceinline__ float cube(const Ar<float>&, float x) { return x * x * x; }
 
 // Model constants in the state type.
 template <typename T> struct P {
@@ -141,75 +169,87 @@ static __device__ __forceinline__ float plus_zero(float t) { return t + 0.0f; }
 //   acc + weight * (yh - 2.0*y + yl), with y2 = 2.0*y precomputed (exact).
 // FIRST marks the first axis, where acc is the initial 0.0.
 template <typename T, bool UNIT_W, bool FIRST = false>
-static __device__ __forceinline__ T lap_axis(T acc, T yh, T y2, T yl, T w)
+static __device__ __forceinline__ T lap_axis(const Ar<T>& A, T acc, T yh, T y2, T yl, T w)
 {
-    using A = Ar<T>;
-    T t = A::add(A::sub(yh, y2), yl);
-    if (!UNIT_W) t = A::mul(w, t);
+    T t = A.add(A.sub(yh, y2), yl);
+    if (!UNIT_W) t = A.mul(w, t);
     if (FIRST) return plus_zero(t);
-    return A::add(acc, t);
+    return A.add(acc, t);
 }
 
 // The whole Laplacian of a DIM-dimensional grid in the reference's axis
 // order (axis 0 first): padded axes X (DIM 3), Y (DIM >= 2), Z.
 template <typename T, bool UNIT_W, int DIM>
-static __device__ __forceinline__ T lap_ref(T y2, T xh, T xl, T yh, T yl, T zh, T zl, T wx, T wy, T wz)
+static __device__ __forceinline__ T lap_ref(const Ar<T>& A, T y2, T xh, T xl, T yh, T yl, T zh, T zl, T wx, T wy, T wz)
 {
     T lap = T(0);
-    if (DIM == 3) lap = lap_axis<T, UNIT_W, true>(lap, xh, y2, xl, wx);
-    if (DIM == 3) lap = lap_axis<T, UNIT_W, false>(lap, yh, y2, yl, wy);
-    if (DIM == 2) lap = lap_axis<T, UNIT_W, true>(lap, yh, y2, yl, wy);
-    if (DIM >= 2) lap = lap_axis<T, UNIT_W, false>(lap, zh, y2, zl, wz);
-    else lap = lap_axis<T, UNIT_W, true>(lap, zh, y2, zl, wz);
+    if (DIM == 3) lap = lap_axis<T, UNIT_W, true>(A, lap, xh, y2, xl, wx);
+    if (DIM == 3) lap = lap_axis<T, UNIT_W, false>(A, lap, yh, y2, yl, wy);
+    if (DIM == 2) lap = lap_axis<T, UNIT_W, true>(A, lap, yh, y2, yl, wy);
+    if (DIM >= 2) lap = lap_axis<T, UNIT_W, false>(A, lap, zh, y2, zl, wz);
+    else lap = lap_axis<T, UNIT_W, true>(A, lap, zh, y2, zl, wz);
     return lap;
 }
 
 // kappa*lap, skipping the multiply when kappa is exactly 1 (1.0*x == x).
 template <typename T>
-static __device__ __forceinline__ T kappa_times(T kappa, T lap)
+static __device__ __forceinline__ T kappa_times(const Ar<T>& A, T kappa, T lap)
 {
-    return kappa == T(1) ? lap : Ar<T>::mul(kappa, lap);
+    return kappa == T(1) ? lap : A.mul(kappa, lap);
 }
 
 // Chemical potential of the Cahn-Hilliard models.
 template <typename T, int MODEL>
-static __device__ __forceinline__ T ch_mu(T phi, T lap, const P<T>& p)
+static __device__ __forceinline__ T ch_mu(const Ar<T>& A, T phi, T lap, const P<T>& p)
 {
-    using A = Ar<T>;
     if (MODEL == MMSP_GPU_CH) {
         // 2.0*phi*(1.0-phi)*(1.0-2.0*phi) - K*lap
         T t2 = twice(phi);
-        T fp = A::mul(A::mul(t2, A::sub(T(1), phi)), A::sub(T(1), t2));
-        return A::sub(fp, kappa_times(p.kappa, lap));
+        T fp = A.mul(A.mul(t2, A.sub(T(A.one), phi)), A.sub(T(A.one), t2));
+        return A.sub(fp, kappa_times(A, p.kappa, lap));
     } else {
         // -r*phi + u*pow(phi,3) - K*lap   (cahn-hilliard.cpp:71)
-        T a = A::add(A::mul(p.neg_r, phi), A::mul(p.u, cube(phi)));
-        return A::sub(a, kappa_times(p.kappa, lap));
+        T a = A.add(A.mul(p.neg_r, phi), A.mul(p.u, cube(A, phi)));
+        return A.sub(a, kappa_times(A, p.kappa, lap));
     }
 }
 
 // New value of one order parameter of the Allen-Cahn models.
 template <typename T, int MODEL>
-static __device__ __forceinline__ T ac_new(T phi, T sum, T lap, const P<T>& p)
+static __device__ __forceinline__ T ac_new(const Ar<T>& A, T phi, T sum, T lap, const P<T>& p)
 {
-    using A = Ar<T>;
     if (MODEL == MMSP_GPU_AC) {
         // phi - dt*L*(-phi + phi*phi*phi + 2.0*gamma*phi*(sum - phi*phi) - kappa*lap)
-        T p2 = A::mul(phi, phi);
-        T p3 = A::mul(p2, phi);
-        T a = A::add(-phi, p3);
-        T g = A::mul(A::mul(p.gamma2, phi), A::sub(sum, p2));
-        T c = A::sub(A::add(a, g), kappa_times(p.kappa, lap));
-        return A::sub(phi, A::mul(p.dtm, c));
+        T p2 = A.mul(phi, phi);
+        T p3 = A.mul(p2, phi);
+        T a = A.add(-phi, p3);
+        T g = A.mul(A.mul(p.gamma2, phi), A.sub(sum, p2));
+        T c = A.sub(A.add(a, g), kappa_times(A, p.kappa, lap));
+        return A.sub(phi, A.mul(p.dtm, c));
     } else if (MODEL == MMSP_GPU_GG || MODEL == MMSP_GPU_ZENER) {
         // phi - dt*(-phi - pow(phi,3) + 2.0*(phi*sum - lap))   (graingrowth.cpp:105, zener.cpp:135)
-        T e = A::add(A::sub(-phi, cube(phi)), twice(A::sub(A::mul(phi, sum), lap)));
-        return A::sub(phi, A::mul(p.dtm, e));
+        T e = A.add(A.sub(-phi, cube(A, phi)), twice(A.sub(A.mul(phi, sum), lap)));
+        return A.sub(phi, A.mul(p.dtm, e));
     } else {
         // phi - dt*M*(-r*phi + u*pow(phi,3) - K*lap)   (allen-cahn.cpp:70)
-        T e = A::sub(A::add(A::mul(p.neg_r, phi), A::mul(p.u, cube(phi))), kappa_times(p.kappa, lap));
-        return A::sub(phi, A::mul(p.dtm, e));
+        T e = A.sub(A.add(A.mul(p.neg_r, phi), A.mul(p.u, cube(A, phi))), kappa_times(A, p.kappa, lap));
+        return A.sub(phi, A.mul(p.dtm, e));
     }
+}
+
+// The constants of the expressions in registers (Ar::reg).
+template <typename T>
+static __device__ __forceinline__ P<T> held(const Ar<T>& A, P<T> p)
+{
+    p.wx = A.reg(p.wx);
+    p.wy = A.reg(p.wy);
+    p.wz = A.reg(p.wz);
+    p.kappa = A.reg(p.kappa);
+    p.dtm = A.reg(p.dtm);
+    p.gamma2 = A.reg(p.gamma2);
+    p.neg_r = A.reg(p.neg_r);
+    p.u = A.reg(p.u);
+    return p;
 }
 
 // Periodic index: any integer onto [0, n), as repeated application of

@@ -52,6 +52,16 @@ static OstP<T> ost_narrow(const Coeffs& c, int dim)
     return p;
 }
 
+// The constants of the expressions in registers (Ar::reg).
+template <typename T>
+static __device__ __forceinline__ OstP<T> held(const Ar<T>& A, OstP<T> p)
+{
+    T* v = &p.wx;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(OstP<T>) / sizeof(T)); i++) v[i] = A.reg(v[i]);
+    return p;
+}
+
 // A thread owns one (y, z) column of the padded axes X, Y, Z and walks it
 // plane by plane.  In-plane offsets are 32-bit (a plane holds fewer than
 // 2^31 cells) and fixed per column, the plane pointers advance once per
@@ -76,9 +86,9 @@ static __device__ __forceinline__ Col column_of(const Geom& g, int y, int z)
 // The Laplacian at plane pointer pc from the rolled X neighbours xh, xl
 // (the reference's operand order: lap_ref).
 template <typename T, int DIM, bool UNIT>
-static __device__ __forceinline__ T lap_col(const T* __restrict__ pc, T c, T xh, T xl, const Col& k, const OstP<T>& p)
+static __device__ __forceinline__ T lap_col(const Ar<T>& A, const T* __restrict__ pc, T c, T xh, T xl, const Col& k, const OstP<T>& p)
 {
-    return lap_ref<T, UNIT, DIM>(twice(c), xh, xl, __ldg(pc + k.yh), __ldg(pc + k.yl), __ldg(pc + k.zh),
+    return lap_ref<T, UNIT, DIM>(A, twice(c), xh, xl, __ldg(pc + k.yh), __ldg(pc + k.yl), __ldg(pc + k.zh),
                                  __ldg(pc + k.zl), p.wx, p.wy, p.wz);
 }
 
@@ -86,16 +96,15 @@ static __device__ __forceinline__ T lap_col(const T* __restrict__ pc, T c, T xh,
 // offset o of plane offset xo.  NF: the field count when it is a
 // compile-time constant (loops unroll), 0 when it is taken from N.
 template <typename T, int NF>
-static __device__ __forceinline__ T order_sum(const T* __restrict__ s, long long xo, int o, long long cells, int N)
+static __device__ __forceinline__ T order_sum(const Ar<T>& A, const T* __restrict__ s, long long xo, int o, long long cells, int N)
 {
-    using A = Ar<T>;
     const int n = NF ? NF : N;
     T sum = T(0);
 #pragma unroll(NF ? NF : 1)
     for (int j = 1; j < (NF ? NF : 64); j++) {
         if (!NF && j >= n) break;
         const T e = __ldg(s + (long long)j * cells + xo + o);
-        sum = j == 1 ? A::mul(e, e) : A::add(sum, A::mul(e, e));
+        sum = j == 1 ? A.mul(e, e) : A.add(sum, A.mul(e, e));
     }
     return sum;
 }
@@ -108,9 +117,10 @@ constexpr int kOstZ = 32, kOstY = 4, kOstPlanes = 8;
 //   w = -A*(C-Cm) + B*pow(C-Cm,3) + Da*pow(C-Ca,3) + Db*pow(C-Cb,3) - g*(C-Ca)*sum - kappa*lap C
 template <typename T, int DIM, bool UNIT, int NF>
 __global__ void __launch_bounds__(kOstZ * kOstY)
-ostwald_mu(const T* __restrict__ s, T* __restrict__ w, Geom g, OstP<T> p, int N)
+ostwald_mu(const T* __restrict__ s, T* __restrict__ w, Geom g, OstP<T> p0, int N)
 {
-    using A = Ar<T>;
+    const Ar<T> A(g.dim);
+    const OstP<T> p = held(A, p0);
     const int z = blockIdx.x * kOstZ + threadIdx.x;
     const int y = blockIdx.y * kOstY + threadIdx.y;
     if (z >= g.Z || y >= g.Y) return;
@@ -124,16 +134,16 @@ ostwald_mu(const T* __restrict__ s, T* __restrict__ w, Geom g, OstP<T> p, int N)
         const T* ph = s + (long long)(x + 1 == g.X ? 0 : x + 1) * YZ;
         const T ch = __ldg(ph + k.o);
         const long long xo = (long long)x * YZ;
-        const T sum = order_sum<T, NF>(s, xo, k.o, g.cells, N);
+        const T sum = order_sum<T, NF>(A, s, xo, k.o, g.cells, N);
         const T C = cc;
-        const T lap = lap_col<T, DIM, UNIT>(pc, cc, ch, cl, k, p);
-        const T dm = A::sub(C, p.Cm), da = A::sub(C, p.Ca), db = A::sub(C, p.Cb);
-        T v = A::mul(p.negA, dm);
-        v = A::add(v, A::mul(p.B, cube(dm)));
-        v = A::add(v, A::mul(p.Da, cube(da)));
-        v = A::add(v, A::mul(p.Db, cube(db)));
-        v = A::sub(v, A::mul(A::mul(p.g, da), sum));
-        w[xo + k.o] = A::sub(v, kappa_times(p.kappa, lap));
+        const T lap = lap_col<T, DIM, UNIT>(A, pc, cc, ch, cl, k, p);
+        const T dm = A.sub(C, p.Cm), da = A.sub(C, p.Ca), db = A.sub(C, p.Cb);
+        T v = A.mul(p.negA, dm);
+        v = A.add(v, A.mul(p.B, cube(A, dm)));
+        v = A.add(v, A.mul(p.Da, cube(A, da)));
+        v = A.add(v, A.mul(p.Db, cube(A, db)));
+        v = A.sub(v, A.mul(A.mul(p.g, da), sum));
+        w[xo + k.o] = A.sub(v, kappa_times(A, p.kappa, lap));
         cl = cc;
         cc = ch;
         pc = ph;
@@ -147,9 +157,10 @@ ostwald_mu(const T* __restrict__ s, T* __restrict__ w, Geom g, OstP<T> p, int N)
 // roll their X neighbours through registers.
 template <typename T, int DIM, bool UNIT, int NF>
 __global__ void __launch_bounds__(kOstZ * kOstY)
-ostwald_update(const T* __restrict__ s, const T* __restrict__ w, T* __restrict__ out, Geom g, OstP<T> p, int N)
+ostwald_update(const T* __restrict__ s, const T* __restrict__ w, T* __restrict__ out, Geom g, OstP<T> p0, int N)
 {
-    using A = Ar<T>;
+    const Ar<T> A(g.dim);
+    const OstP<T> p = held(A, p0);
     constexpr int NE = NF ? NF - 1 : 1;   // order parameters rolled (none when NF is 0)
     const int z = blockIdx.x * kOstZ + threadIdx.x;
     const int y = blockIdx.y * kOstY + threadIdx.y;
@@ -173,20 +184,20 @@ ostwald_update(const T* __restrict__ s, const T* __restrict__ w, T* __restrict__
         const long long xho = (long long)(x + 1 == g.X ? 0 : x + 1) * YZ;
         const T wh = __ldg(w + xho + k.o);
         const T C = __ldg(s + xo + k.o);
-        out[xo + k.o] = A::add(C, A::mul(p.dtD, lap_col<T, DIM, UNIT>(wc_p, wc, wh, wl, k, p)));
-        const T sum = order_sum<T, NF>(s, xo, k.o, cells, N);
-        const T da = A::sub(C, p.Ca);
-        const T t1 = A::mul(p.neg_g, A::mul(da, da));
+        out[xo + k.o] = A.add(C, A.mul(p.dtD, lap_col<T, DIM, UNIT>(A, wc_p, wc, wh, wl, k, p)));
+        const T sum = order_sum<T, NF>(A, s, xo, k.o, cells, N);
+        const T da = A.sub(C, p.Ca);
+        const T t1 = A.mul(p.neg_g, A.mul(da, da));
         if (NF) {
 #pragma unroll
             for (int j = 0; j < NE; j++) {
                 const T* f = s + (long long)(j + 1) * cells;
                 const T e = ec[j];
                 const T eh = __ldg(f + xho + k.o);
-                T v = A::add(t1, A::mul(p.delta, cube(e)));
-                v = A::add(v, A::mul(A::mul(p.eps, e), A::sub(sum, A::mul(e, e))));
-                v = A::sub(v, kappa_times(p.kappa, lap_col<T, DIM, UNIT>(f + xo, e, eh, el[j], k, p)));
-                out[(long long)(j + 1) * cells + xo + k.o] = A::sub(e, A::mul(p.dtL, v));
+                T v = A.add(t1, A.mul(p.delta, cube(A, e)));
+                v = A.add(v, A.mul(A.mul(p.eps, e), A.sub(sum, A.mul(e, e))));
+                v = A.sub(v, kappa_times(A, p.kappa, lap_col<T, DIM, UNIT>(A, f + xo, e, eh, el[j], k, p)));
+                out[(long long)(j + 1) * cells + xo + k.o] = A.sub(e, A.mul(p.dtL, v));
                 el[j] = e;
                 ec[j] = eh;
             }
@@ -195,11 +206,11 @@ ostwald_update(const T* __restrict__ s, const T* __restrict__ w, T* __restrict__
             for (int j = 1; j < N; j++) {
                 const T* f = s + (long long)j * cells;
                 const T e = __ldg(f + xo + k.o);
-                T v = A::add(t1, A::mul(p.delta, cube(e)));
-                v = A::add(v, A::mul(A::mul(p.eps, e), A::sub(sum, A::mul(e, e))));
-                v = A::sub(v, kappa_times(p.kappa, lap_col<T, DIM, UNIT>(f + xo, e, __ldg(f + xho + k.o),
+                T v = A.add(t1, A.mul(p.delta, cube(A, e)));
+                v = A.add(v, A.mul(A.mul(p.eps, e), A.sub(sum, A.mul(e, e))));
+                v = A.sub(v, kappa_times(A, p.kappa, lap_col<T, DIM, UNIT>(A, f + xo, e, __ldg(f + xho + k.o),
                                                                         __ldg(f + xlo2 + k.o), k, p)));
-                out[(long long)j * cells + xo + k.o] = A::sub(e, A::mul(p.dtL, v));
+                out[(long long)j * cells + xo + k.o] = A.sub(e, A.mul(p.dtL, v));
             }
         }
         wl = wc;

@@ -86,6 +86,7 @@ sparse_gg_step(SpView in, SpView out, Geom g, SpConst q, int K, int* __restrict_
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.cells) return;
     const long long cells = g.cells;
+    const Ar<double> A(g.dim);
     // padded coordinates and the periodic face neighbours of the real axes,
     // in the reference's axis order (real axis 0 first)
     const int x = (int)(c / g.YZ);
@@ -137,7 +138,7 @@ sparse_gg_step(SpView in, SpView out, Geom g, SpConst q, int K, int* __restrict_
         double sum = 0.0;
         for (int h = 0; h < own; h++) {
             const double phi = __ldg(in.val + h * cells + c);
-            sum = __dadd_rn(sum, __dmul_rn(phi, phi));
+            sum = A.add(sum, A.mul(phi, phi));
         }
         // newGrid(n) as it stands: the state of two steps back
         int dn = out.cnt[c];
@@ -148,11 +149,11 @@ sparse_gg_step(SpView in, SpView out, Geom g, SpConst q, int K, int* __restrict_
             double lap = 0.0;
 #pragma unroll
             for (int ra = 0; ra < DIM; ra++) {
-                double t = __dadd_rn(__dsub_rn(sp_get(in, cells, hi[ra], i), y2), sp_get(in, cells, lo[ra], i));
-                if (!UNIT) t = __dmul_rn(q.w[ra], t);
-                lap = ra == 0 ? plus_zero(t) : __dadd_rn(lap, t);
+                double t = A.add(A.sub(sp_get(in, cells, hi[ra], i), y2), sp_get(in, cells, lo[ra], i));
+                if (!UNIT) t = A.mul(q.w[ra], t);
+                lap = ra == 0 ? plus_zero(t) : A.add(lap, t);
             }
-            const double v = ac_new<double, MMSP_GPU_GG>(phi, sum, lap, q.p);
+            const double v = ac_new<double, MMSP_GPU_GG>(A, phi, sum, lap, q.p);
             if (v > q.eps) {
                 int h = 0;
                 while (h < dn && out.idx[h * cells + c] != i) h++;
