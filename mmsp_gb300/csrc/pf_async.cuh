@@ -25,13 +25,6 @@ static __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
 
-// Arrive on `bar` (release: this thread's earlier shared-memory accesses
-// are ordered before the phase completes).
-static __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // Make initialised barriers visible to the asynchronous proxy.
 static __device__ __forceinline__ void mbar_fence_init()
 {
@@ -112,13 +105,6 @@ static __device__ __forceinline__ void cp_async4(void* dst, const void* src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
-// Per-thread asynchronous 8-byte copy global -> shared (both addresses
-// 8-byte aligned).
-static __device__ __forceinline__ void cp_async8(void* dst, const void* src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
 // Per-thread asynchronous 16-byte copy global -> shared (both addresses
 // 16-byte aligned), cached in L2 only.
 static __device__ __forceinline__ void cp_async16(void* dst, const void* src)
@@ -130,13 +116,6 @@ static __device__ __forceinline__ void cp_async16(void* dst, const void* src)
 static __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Arrive on `bar` once this thread's earlier cp.async copies have landed; the
-// barrier's expected count must include one arrival per calling thread.
-static __device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
-{
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 }  // namespace pf

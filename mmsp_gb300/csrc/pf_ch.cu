@@ -173,6 +173,7 @@ cudaError_t plan_ch(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
     // otherwise (a 2D rows block holds a whole row: 1024-thread blocks leave
     // the noise arithmetic short of warps), both of which add the noise term
     if (!noisy(d) && ch3_stream_eligible(d, g)) return plan_ch3_stream(d, g, p);
+    if (ch3_flat_eligible(d, g)) return plan_ch3_flat(d, g, p);
     if (ch_rows_eligible(d, g) && (!noisy(d) || g.dim == 3)) return plan_ch_rows(d, g, p);
     p->kind = 0;
     Coeffs c = make_coeffs(d);
@@ -215,6 +216,7 @@ cudaError_t plan_ch(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
 cudaError_t launch_ch(const StepPlan& p, const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c,
                       const void* in, void* out, int* err, cudaStream_t s)
 {
+    if (p.kind == 2) return launch_ch3_flat(p, g, c, in, out, s);
     if (p.kind == 1) return launch_ch3_stream(p, g, c, in, out, err, s);
     if (p.kind == 3) return launch_ch_rows(p, d, c, in, out, err, s);
     int planes = p.planes;

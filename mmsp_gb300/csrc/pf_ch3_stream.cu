@@ -1,28 +1,19 @@
-// pf_ch3_stream.cu -- FP32 3D Cahn-Hilliard step, register streaming along X.
+// pf_ch3_stream.cu -- FP32 3D Cahn-Hilliard step on rows of 256 cells, register streaming along X.
 //
-// The precision-form kernel for 3D grids whose rows (axis Z) hold an even
-// number of cells up to 512.  A block owns R consecutive rows (axis Y) of
-// full Z extent and a run of X planes; each thread owns V adjacent cells of
-// a row (V = 1 for 32-cell rows, else 2), so the block has Z/V threads,
-// rounded up to whole warps (the threads past the row's end compute on
-// copies of its last cells and store nothing).
+// A block owns R consecutive rows (axis Y) of full Z extent and a run of X
+// planes; each thread owns two adjacent cells of a row.
 //
 // For every plane the block's R+4 rows (2 halo rows on each side, wrapped
-// periodically) arrive in shared memory on an mbarrier ring, several planes
-// ahead of the one being computed: by cp.async.bulk where rows are 16-byte
-// multiples, or rows of 2 mod 4 cells on an even number of rows (every
-// copied piece then starts on an even row and spans an even number of
-// rows), by per-thread 8-byte cp.async otherwise.  Each thread keeps its
+// periodically) arrive in shared memory by cp.async.bulk on an mbarrier ring,
+// several planes ahead of the one being computed.  Each thread keeps its
 // cells of c for planes x, x+1, x+2 and of mu for x-1, x, x+1 in registers:
 // Y neighbours are neighbouring registers, X neighbours the neighbouring
 // planes' registers, Z neighbours inside a thread are registers, Z
 // neighbours across threads come from shared memory (c) or warp shuffles
 // (mu), and the first and last cells of each warp exchange mu through a small
-// shared array that wraps periodically across the row (the last warp's last
-// cell is the row's last cell, wherever the row ends in that warp).  mu is
-// recomputed only on the 2 halo rows of the strip; a block spans whole rows,
-// so there is no Z halo.  Rows of 32..512 cells in powers of two have
-// compile-time instances (row offsets become immediates).
+// shared array that wraps periodically across the row.  mu is recomputed only
+// on the 2 halo rows of the strip; a block spans whole rows, so there is no Z
+// halo.
 //
 // FP32 arithmetic is reassociated for throughput (six-neighbour sums and
 // Horner's form of f'(c)); the result is checked against the FP64 oracle
@@ -36,83 +27,52 @@
 
 namespace pf {
 
-#ifndef PF_CH3_RING
-#define PF_CH3_RING 4
-#endif
-#ifndef PF_CH3_MINB
-#define PF_CH3_MINB 3
-#endif
-#ifndef PF_CH3_R
-#define PF_CH3_R 8
-#endif
-constexpr int kRing = PF_CH3_RING;   // planes staged in shared memory (kRing-1 in flight)
-constexpr int kStreamR = PF_CH3_R;   // rows per block strip
+constexpr int kRing = 4;      // planes staged in shared memory (kRing-1 in flight)
+constexpr int kStreamR = 8;   // rows per block strip
 
 struct F32Coef {
     float wx, wy, wz, w2;   // Laplacian weights, w2 = 2(wx+wy+wz)
     float kappa, dtm, neg_r, u;
 };
 
-// A thread's cells: float (one cell) or float2 (two adjacent cells).  float2
-// arithmetic uses the packed FP32x2 instructions, one instruction for both
-// cells.
-template <int V> struct Cells;
-template <> struct Cells<1> { using type = float; };
-template <> struct Cells<2> { using type = float2; };
-
-static __device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+// A thread's two adjacent cells: packed FP32x2 arithmetic, one instruction for both.
 static __device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-static __device__ __forceinline__ float vmul(float a, float b) { return a * b; }
 static __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-static __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 static __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-template <typename VT> static __device__ __forceinline__ VT vset(float k);
-template <> __device__ __forceinline__ float vset<float>(float k) { return k; }
-template <> __device__ __forceinline__ float2 vset<float2>(float k) { return make_float2(k, k); }
-static __device__ __forceinline__ float vfirst(float a) { return a; }
-static __device__ __forceinline__ float vfirst(float2 a) { return a.x; }
-static __device__ __forceinline__ float vlast(float a) { return a; }
-static __device__ __forceinline__ float vlast(float2 a) { return a.y; }
+static __device__ __forceinline__ float2 vset(float k) { return make_float2(k, k); }
 // Sum of the two Z neighbours of each cell, given the cells just left and
-// just right of the thread's run.
-static __device__ __forceinline__ float vzsum(float, float left, float right) { return left + right; }
+// just right of the thread's pair.
 static __device__ __forceinline__ float2 vzsum(float2 c, float left, float right)
 {
     return __fadd2_rn(make_float2(left, c.x), make_float2(c.y, right));
 }
 
-template <int MODEL, typename VT>
-static __device__ __forceinline__ VT mu_v(VT c, VT lap, const F32Coef& q)
+template <int MODEL>
+static __device__ __forceinline__ float2 mu_v(float2 c, float2 lap, const F32Coef& q)
 {
-    VT fp;
+    float2 fp;
     if (MODEL == MMSP_GPU_CH)   // 2c(1-c)(1-2c) = c*(2 + c*(-6 + 4c))
-        fp = vmul(c, vfma(vfma(vset<VT>(4.0f), c, vset<VT>(-6.0f)), c, vset<VT>(2.0f)));
+        fp = vmul(c, vfma(vfma(vset(4.0f), c, vset(-6.0f)), c, vset(2.0f)));
     else                        // -r c + u c^3 = c*(u c^2 - r)
-        fp = vmul(c, vfma(vset<VT>(q.u), vmul(c, c), vset<VT>(q.neg_r)));
-    return vfma(vset<VT>(-q.kappa), lap, fp);
+        fp = vmul(c, vfma(vset(q.u), vmul(c, c), vset(q.neg_r)));
+    return vfma(vset(-q.kappa), lap, fp);
 }
 
 // wx*sx + wy*sy + wz*sz - 2(wx+wy+wz)*c, with sx, sy, sz the sums of the two
 // neighbours along each axis.
-template <bool UNIT, typename VT>
-static __device__ __forceinline__ VT lap_v(VT sx, VT sy, VT sz, VT c, const F32Coef& q)
+template <bool UNIT>
+static __device__ __forceinline__ float2 lap_v(float2 sx, float2 sy, float2 sz, float2 c, const F32Coef& q)
 {
-    if (UNIT) return vfma(vset<VT>(-6.0f), c, vadd(vadd(sx, sy), sz));
-    return vfma(vset<VT>(q.wx), sx, vfma(vset<VT>(q.wy), sy, vfma(vset<VT>(q.wz), sz, vmul(vset<VT>(-q.w2), c))));
+    if (UNIT) return vfma(vset(-6.0f), c, vadd(vadd(sx, sy), sz));
+    return vfma(vset(q.wx), sx, vfma(vset(q.wy), sy, vfma(vset(q.wz), sz, vmul(vset(-q.w2), c))));
 }
 
-// Threads of a block for rows of Z cells, V per thread: whole warps.
-static int ch3_threads(int Z, int V) { return ((Z + V - 1) / V + 31) / 32 * 32; }
-
-// Shared memory: kRing slots of (R+4) x ZS floats (ZS the shared row
-// stride: Z, Z + 1 for odd rows of two cells per thread, or the instance's
-// full TM*V row), the warp-end mu buffers [parity][warp][side][R], then
-// kRing mbarriers.
-static size_t ch3_smem(int R, int Z, int V, int ZS)
+// Shared memory: kRing slots of (R+4) x Z floats, the warp-end mu buffers
+// [parity][warp][side][R], then kRing mbarriers.
+static size_t ch3_smem(int R, int Z)
 {
-    const int warps = ch3_threads(Z, V) / 32;
-    return sizeof(float) * (size_t)kRing * (R + 4) * ZS + sizeof(float) * 2 * warps * 2 * R +
-           sizeof(uint64_t) * kRing;
+    const int warps = Z / 64;
+    return sizeof(float) * (size_t)kRing * (R + 4) * Z + sizeof(float) * 2 * warps * 2 * R + sizeof(uint64_t) * kRing;
 }
 
 // STALL: the failure-detection test (never in normal use).  The plane fills
@@ -120,43 +80,20 @@ static size_t ch3_smem(int R, int Z, int V, int ZS)
 // 4 polls, so the waits run out with no copy in flight and the launch takes
 // its timed-out exit (error word, bounded drain, return).  The host selects
 // it only through MMSP_GPU_TEST_STALL_LAUNCHES.
-// ZT: the row length when it is a compile-time constant (32..512 in powers
-// of two, ZT / V = TM threads), 0 when it is taken from the grid
-// (blockDim.x = ch3_threads(Z, V) <= TM).  BULK: the pieces of a plane's
-// strip are 16-byte aligned (rows of a multiple of 4 cells, or of 2 mod 4
-// cells with Y even) and thread 0 stages each plane with cp.async.bulk (one
-// arrival, transaction-counted); otherwise every thread copies its cells
-// with 4- or 8-byte cp.async and arrives when they land.  PAD: odd rows of
-// two cells per thread: shared rows hold Z + 1 cells, the extra one a copy
-// of the row's cell 0 (the periodic right neighbour of the last cell), the
-// last thread takes mu of cell 0 from the warp-end exchange for its second
-// cell, and stores are 4-byte (odd rows break 8-byte alignment).  WIDE
-// (with per-thread copies): shared rows are TM*V floats apart whatever Z
-// is, so shared offsets are compile-time.
-template <int R, int ZT, int TM, int V, int MODEL, bool UNIT, bool STALL, bool BULK, bool PAD, bool WIDE>
-__global__ void __launch_bounds__(TM, TM <= 128 ? PF_CH3_MINB : (V == 1 && TM == 256 ? 2 : 1))
+template <int R, int Z, int MODEL, bool UNIT, bool STALL>
+__global__ void __launch_bounds__(Z / 2, 3)
 ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, F32Coef q, int planes,
-               int* __restrict__ err)
+               int mirror, int* __restrict__ err)
 {
-    constexpr int RR = R + 4;
-    static_assert(TM % 32 == 0 && R % 4 == 0 && (!ZT || ZT == TM * V), "row split");
-    static_assert(!PAD || (V == 2 && !ZT && !BULK), "odd rows: runtime rows, per-thread copies");
-    static_assert(!WIDE || (!ZT && !BULK), "full-width shared rows: runtime rows, per-thread copies");
-    const int Z = ZT ? ZT : g.Z;
-    // shared-memory row stride: a compile-time TM*V for WIDE instances, so
-    // every shared address in the plane loop is an immediate offset
-    const int ZS = WIDE ? TM * V : PAD ? Z + 1 : Z;
-    const int W = ZT ? TM / 32 : (int)(blockDim.x >> 5);   // warps per block
+    constexpr int RR = R + 4, V = 2, TM = Z / V, W = TM / 32;   // threads and warps per block
+    static_assert(TM % 32 == 0 && R % 4 == 0, "row split");
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
-    const int tl = (Z + V - 1) / V - 1;  // the thread holding the row's last cells
-    const bool real = ZT || t <= tl;     // past the row's end: compute on the last cells, store nothing
-    const int z0 = (real ? t : tl) * V;  // first cell of this thread
-    const int wlast = W - 1;             // (whole warps: the last warp holds the row's last cells)
-    const int lane_last = warp == wlast ? (ZT ? 31 : tl & 31) : 31;   // this warp's last real lane
+    const int z0 = t * V;        // first cell of this thread
+    const int wlast = W - 1;
     extern __shared__ __align__(128) unsigned char sm[];
     float* slots = reinterpret_cast<float*>(sm);
-    float* edges = slots + (size_t)kRing * RR * ZS;
+    float* edges = slots + (size_t)kRing * RR * Z;
     uint64_t* bars = reinterpret_cast<uint64_t*>(edges + 2 * W * 2 * R);
     __shared__ int s_err;
 
@@ -165,54 +102,39 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
     const int xe = min(xs + planes, g.X);
     if (xs >= xe) return;
     const int zl = z0 == 0 ? Z - 1 : z0 - 1;            // cell left of this thread's first
-    // cell right of this thread's last (PAD: the last thread's second cell is
-    // the copy of cell 0, and its right neighbour, unused, is any cell)
-    const int zh = z0 + V >= Z ? z0 + V - Z : z0 + V;
+    const int zh = z0 + V == Z ? 0 : z0 + V;            // cell right of its last
     const int wl = warp == 0 ? wlast : warp - 1;
     const int wh = warp == wlast ? 0 : warp + 1;
     const int x_first = xs - 2, x_last = xe + 1;        // planes read from global memory
 
-    // stage plane pl (wrapped) into its ring slot: thread 0 (BULK) or every thread
+    // stage plane pl (wrapped) into its ring slot: thread 0
     auto fill = [&](int pl) {
         const int k = pl - x_first, s = k % kRing;
         uint64_t* bar = &bars[s];
-        float* dst = slots + (size_t)s * RR * ZS;
-        const float* base = cin + (long long)wrapi(pl, g.X) * g.YZ;
-        if constexpr (BULK) {
-            const uint32_t row = (uint32_t)Z * sizeof(float);
-            fence_proxy_async();
-            mbar_expect_tx(bar, RR * row);
-            if (STALL) return;   // failure-detection test: the bytes never arrive
-            const int a = y0 - 2, b = y0 + R + 2;
-            if (a >= 0 && b <= g.Y) {
-                bulk_g2s(dst, base + (long long)a * Z, RR * row, bar);
-            } else if (a < 0) {
-                const int n1 = -a;   // rows Y-n1 .. Y-1 first, then 0 ..
-                bulk_g2s(dst, base + (long long)(g.Y - n1) * Z, n1 * row, bar);
-                bulk_g2s(dst + n1 * Z, base, (RR - n1) * row, bar);
-            } else {
-                const int n1 = g.Y - a;   // rows a .. Y-1, then 0 ..
-                bulk_g2s(dst, base + (long long)a * Z, n1 * row, bar);
-                bulk_g2s(dst + n1 * Z, base, (RR - n1) * row, bar);
-            }
+        float* dst = slots + (size_t)s * RR * Z;
+        // mirror: the walk runs through X downwards.  Successive steps
+        // alternate, so a step starts with the planes that the one before
+        // touched last, which are still in L2.
+        const int xw = wrapi(pl, g.X);
+        const float* base = cin + (long long)(mirror ? g.X - 1 - xw : xw) * g.YZ;
+        const uint32_t row = (uint32_t)Z * sizeof(float);
+        fence_proxy_async();
+        mbar_expect_tx(bar, RR * row);
+        if (STALL) return;   // failure-detection test: the bytes never arrive
+        const int a = y0 - 2, b = y0 + R + 2;
+        if (a >= 0 && b <= g.Y) {
+            bulk_g2s(dst, base + (long long)a * Z, RR * row, bar);
+        } else if (a < 0) {
+            const int n1 = -a;   // rows Y-n1 .. Y-1 first, then 0 ..
+            bulk_g2s(dst, base + (long long)(g.Y - n1) * Z, n1 * row, bar);
+            bulk_g2s(dst + n1 * Z, base, (RR - n1) * row, bar);
         } else {
-            if (STALL) return;   // no copies and no arrivals: the waits run out
-            if (real)
-                for (int i = 0; i < RR; i++) {
-                    const float* row = base + (long long)wrap_near(y0 - 2 + i, g.Y) * Z;   // g.Y >= R + 4
-                    if (PAD) {   // 4-byte copies: odd rows break 8-byte alignment; cell Z is cell 0
-                        cp_async4(dst + i * ZS + z0, row + z0);
-                        cp_async4(dst + i * ZS + z0 + 1, row + (z0 + 1 == Z ? 0 : z0 + 1));
-                    } else if (V == 2) {
-                        cp_async8(dst + i * ZS + z0, row + z0);
-                    } else {
-                        cp_async4(dst + i * ZS + z0, row + z0);
-                    }
-                }
-            cp_async_arrive(bar);
+            const int n1 = g.Y - a;   // rows a .. Y-1, then 0 ..
+            bulk_g2s(dst, base + (long long)a * Z, n1 * row, bar);
+            bulk_g2s(dst + n1 * Z, base, (RR - n1) * row, bar);
         }
     };
-    auto slot_of = [&](int pl) -> const float* { return slots + (size_t)((pl - x_first) % kRing) * RR * ZS; };
+    auto slot_of = [&](int pl) -> const float* { return slots + (size_t)((pl - x_first) % kRing) * RR * Z; };
     auto wait_plane = [&](int pl) {
         const int k = pl - x_first;
         if (!mbar_wait(&bars[k % kRing], (uint32_t)(k / kRing) & 1u, STALL ? 4u : kSpinLimit)) {
@@ -222,15 +144,15 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
     };
 
     if (t == 0) {
-        for (int s = 0; s < kRing; s++) mbar_init(&bars[s], BULK ? 1 : (int)blockDim.x);
+        for (int s = 0; s < kRing; s++) mbar_init(&bars[s], 1);
         mbar_fence_init();
         s_err = 0;
     }
     __syncthreads();
-    if (!BULK || t == 0)   // (evaluated where used: a flag held across the loop costs registers)
+    if (t == 0)
         for (int pl = x_first; pl < x_first + kRing && pl <= x_last; pl++) fill(pl);
 
-    using VT = typename Cells<V>::type;
+    using VT = float2;
     VT cA[RR], cB[RR], cC[RR];
     VT mA[R + 2], mB[R + 2], mC[R + 2];
     wait_plane(x_first);
@@ -240,14 +162,14 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
         const float* s1 = slot_of(x_first + 1) + z0;
 #pragma unroll
         for (int i = 0; i < RR; i++) {
-            cA[i] = *reinterpret_cast<const VT*>(s0 + i * ZS);
-            cB[i] = *reinterpret_cast<const VT*>(s1 + i * ZS);
+            cA[i] = *reinterpret_cast<const VT*>(s0 + i * Z);
+            cB[i] = *reinterpret_cast<const VT*>(s1 + i * Z);
         }
     }
 #pragma unroll
-    for (int i = 0; i < R + 2; i++) mA[i] = mB[i] = vset<VT>(0.0f);
+    for (int i = 0; i < R + 2; i++) mA[i] = mB[i] = vset(0.0f);
     __syncthreads();
-    if ((!BULK || t == 0) && !s_err && x_first + kRing <= x_last) fill(x_first + kRing);   // slot of x_first is free
+    if (t == 0 && !s_err && x_first + kRing <= x_last) fill(x_first + kRing);   // slot of x_first is free
 
     // One plane: a = c(x), b = c(x+1), c = c(x+2) (loaded here); ma = mu(x-1),
     // mb = mu(x), mc = mu(x+1) (computed here); writes c'(x) when x >= xs.
@@ -256,13 +178,13 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
         wait_plane(x + 2);
         const float* s2 = slot_of(x + 2) + z0;
 #pragma unroll
-        for (int i = 0; i < RR; i++) c[i] = *reinterpret_cast<const VT*>(s2 + i * ZS);
+        for (int i = 0; i < RR; i++) c[i] = *reinterpret_cast<const VT*>(s2 + i * Z);
         const float* s1 = slot_of(x + 1);
 #pragma unroll
         for (int r = -1; r <= R; r++) {
             const int i = r + 2;
-            const float left = s1[i * ZS + zl];
-            const float right = s1[i * ZS + zh];
+            const float left = s1[i * Z + zl];
+            const float right = s1[i * Z + zh];
             const VT cc = b[i];
             const VT lap = lap_v<UNIT>(vadd(a[i], c[i]), vadd(b[i - 1], b[i + 1]), vzsum(cc, left, right), cc, q);
             mc[r + 1] = mu_v<MODEL>(cc, lap, q);
@@ -270,36 +192,15 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
         // warp ends publish mu(x+1) of rows 0..R-1 for the neighbouring warps:
         // lane 0 its first cell, the warp's last real lane its last
         float* e1 = edges + (((x + 1) & 1) * W + warp) * 2 * R;
-        if (ZT) {
-            if (lane == 0 || lane == 31) {
-                // (selects keep mc in registers)
-                const bool first = lane == 0;
-                float* dst = e1 + (first ? 0 : R);
+        if (lane == 0 || lane == 31) {
+            // (selects keep mc in registers)
+            const bool first = lane == 0;
+            float* dst = e1 + (first ? 0 : R);
 #pragma unroll
-                for (int r = 0; r < R; r += 4)
-                    *reinterpret_cast<float4*>(dst + r) = make_float4(
-                        first ? vfirst(mc[r + 1]) : vlast(mc[r + 1]), first ? vfirst(mc[r + 2]) : vlast(mc[r + 2]),
-                        first ? vfirst(mc[r + 3]) : vlast(mc[r + 3]), first ? vfirst(mc[r + 4]) : vlast(mc[r + 4]));
-            }
-        } else {
-            if (lane == 0)
-#pragma unroll
-                for (int r = 0; r < R; r += 4)
-                    *reinterpret_cast<float4*>(e1 + r) = make_float4(vfirst(mc[r + 1]), vfirst(mc[r + 2]),
-                                                                     vfirst(mc[r + 3]), vfirst(mc[r + 4]));
-            if (lane == lane_last) {   // (PAD: the row's last real cell is the first of its pair)
-                if (PAD && warp == wlast) {
-#pragma unroll
-                    for (int r = 0; r < R; r += 4)
-                        *reinterpret_cast<float4*>(e1 + R + r) = make_float4(vfirst(mc[r + 1]), vfirst(mc[r + 2]),
-                                                                             vfirst(mc[r + 3]), vfirst(mc[r + 4]));
-                } else {
-#pragma unroll
-                    for (int r = 0; r < R; r += 4)
-                        *reinterpret_cast<float4*>(e1 + R + r) = make_float4(vlast(mc[r + 1]), vlast(mc[r + 2]),
-                                                                             vlast(mc[r + 3]), vlast(mc[r + 4]));
-                }
-            }
+            for (int r = 0; r < R; r += 4)
+                *reinterpret_cast<float4*>(dst + r) = make_float4(
+                    first ? mc[r + 1].x : mc[r + 1].y, first ? mc[r + 2].x : mc[r + 2].y,
+                    first ? mc[r + 3].x : mc[r + 3].y, first ? mc[r + 4].x : mc[r + 4].y);
         }
         if (x >= xs) {
             // the neighbouring warps' end cells: every lane reads the same
@@ -313,34 +214,23 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
                 el[r] = u.x, el[r + 1] = u.y, el[r + 2] = u.z, el[r + 3] = u.w;
                 eh[r] = v.x, eh[r + 1] = v.y, eh[r + 2] = v.z, eh[r + 3] = v.w;
             }
-            float* dst = cout + (long long)x * g.YZ + (long long)y0 * Z + z0;
+            float* dst = cout + (long long)(mirror ? g.X - 1 - x : x) * g.YZ + (long long)y0 * Z + z0;
             const int rows = min(R, g.Y - y0);
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const float up = __shfl_up_sync(0xffffffffu, vlast(mb[r + 1]), 1);
-                const float down = __shfl_down_sync(0xffffffffu, vfirst(mb[r + 1]), 1);
-                const float left = lane == 0 ? el[r] : up;
-                const float right = lane == lane_last ? eh[r] : down;
                 const VT m = mb[r + 1];
-                VT mz = m;   // PAD, last thread: the second cell's mu is that of cell 0
-                if constexpr (PAD) {
-                    if (warp == wlast && lane == lane_last) mz.y = eh[r];
-                }
-                const VT lap = lap_v<UNIT>(vadd(ma[r + 1], mc[r + 1]), vadd(mb[r], mb[r + 2]), vzsum(mz, left, right), m, q);
-                const VT o = vfma(vset<VT>(q.dtm), lap, a[r + 2]);
-                if constexpr (PAD) {
-                    if (r < rows && real) {
-                        dst[(long long)r * Z] = vfirst(o);
-                        if (z0 + 1 < Z) dst[(long long)r * Z + 1] = vlast(o);
-                    }
-                } else {
-                    if (r < rows && real) *reinterpret_cast<VT*>(dst + (long long)r * Z) = o;
-                }
+                const float up = __shfl_up_sync(0xffffffffu, m.y, 1);
+                const float down = __shfl_down_sync(0xffffffffu, m.x, 1);
+                const float left = lane == 0 ? el[r] : up;
+                const float right = lane == 31 ? eh[r] : down;
+                const VT lap = lap_v<UNIT>(vadd(ma[r + 1], mc[r + 1]), vadd(mb[r], mb[r + 2]), vzsum(m, left, right), m, q);
+                const VT o = vfma(vset(q.dtm), lap, a[r + 2]);
+                if (r < rows) *reinterpret_cast<VT*>(dst + (long long)r * Z) = o;
             }
         }
         __syncthreads();
         if (s_err) return false;
-        if ((!BULK || t == 0) && x + 1 + kRing <= x_last) fill(x + 1 + kRing);   // slot of x+1 is free now
+        if (t == 0 && x + 1 + kRing <= x_last) fill(x + 1 + kRing);   // slot of x+1 is free now
         return true;
     };
 
@@ -353,10 +243,8 @@ ch3_stream_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, 
         if (x >= xe || !iter(x, cC, cA, cB, mC, mA, mB)) break;
         x++;
     }
-    if (s_err && (!BULK || t == 0)) {
+    if (s_err && t == 0) {
         // leave no copy in flight: wait (bounded) for every issued fill
-        // (per-thread copies: every thread waits for its own)
-        if (!BULK) cp_async_wait_all();
         for (int pl = max(x, x_first); pl <= min(x + kRing, x_last); pl++) {
             const int k = pl - x_first;
             mbar_wait(&bars[k % kRing], (uint32_t)(k / kRing) & 1u, STALL ? 4u : kSpinLimit);
@@ -379,90 +267,63 @@ static F32Coef f32coef(const Coeffs& c)
 }
 
 // MMSP_GPU_TEST_STALL_LAUNCHES=n: the next n launches of this kernel in the
-// process run its STALL form (the failure-detection test).  Read once; unset
-// in normal use.
+// process run its STALL form, and grids with rows of 64 cells take this
+// kernel too (the failure-detection test).  Read once; unset in normal use.
 static std::atomic<int> g_stall_left{-1};
-static int take_stall()
+static int stall_left()
 {
     int left = g_stall_left.load();
     if (left < 0) {
         const char* v = getenv("MMSP_GPU_TEST_STALL_LAUNCHES");
         int n = v ? atoi(v) : 0;
         g_stall_left.compare_exchange_strong(left, n > 0 ? n : 0);
+        left = g_stall_left.load();
     }
-    int cur = g_stall_left.load();
+    return left;
+}
+static int take_stall()
+{
+    int cur = stall_left();
     while (cur > 0 && !g_stall_left.compare_exchange_weak(cur, cur - 1)) {
     }
     return cur > 0 ? 1 : 0;
 }
 
-// cells per thread: 2 (packed FP32x2), 1 for 32-cell rows
-static int cells_per_thread(int Z) { return Z == 32 ? 1 : 2; }
-
+// Rows of 256 cells whose two states fill L2 or do not fit it: there the
+// ring's bulk copies keep more of HBM and L2 busy than the loads of
+// pf_ch3_flat.cu.  us per step, here / there: 256^3 (128 MB) 24.9 / 28.7,
+// 512x256x256 45.0 / 52.5, 200x256x256 (100 MB) 20.5 / 23.9, 160x256x256 (80
+// MB) 17.2 / 18.2; 128x256x256 (64 MB) 14.9 / 14.2.  Every other row length is
+// faster there.
+constexpr long long kStreamL2 = 72LL << 20;
 bool ch3_stream_eligible(const mmsp_gpu_desc& d, const Geom& g)
 {
-    return d.dtype == MMSP_GPU_F32 && g.dim == 3 && g.Z >= 32 && g.Z <= 512 && g.Y >= kStreamR + 4 &&
-           (d.model == MMSP_GPU_CH || d.model == MMSP_GPU_CH_POLY);
+    const bool ch = d.dtype == MMSP_GPU_F32 && g.dim == 3 && g.Y >= kStreamR + 4 &&
+                    (d.model == MMSP_GPU_CH || d.model == MMSP_GPU_CH_POLY);
+    return ch && ((g.Z == 256 && 8LL * g.cells > kStreamL2) || (g.Z == 64 && stall_left() > 0));
 }
 
-template <int ZT, int TM, int V, bool STALL, bool BULK, bool PAD = false, bool WIDE = false>
-static const void* pick_mu(bool ch, bool unit)
+template <int Z, bool STALL>
+static const void* pick_stream(bool ch, bool unit)
 {
     if (ch)
-        return unit ? (const void*)&ch3_stream_f32<kStreamR, ZT, TM, V, MMSP_GPU_CH, true, STALL, BULK, PAD, WIDE>
-                    : (const void*)&ch3_stream_f32<kStreamR, ZT, TM, V, MMSP_GPU_CH, false, STALL, BULK, PAD, WIDE>;
-    return unit ? (const void*)&ch3_stream_f32<kStreamR, ZT, TM, V, MMSP_GPU_CH_POLY, true, STALL, BULK, PAD, WIDE>
-                : (const void*)&ch3_stream_f32<kStreamR, ZT, TM, V, MMSP_GPU_CH_POLY, false, STALL, BULK, PAD, WIDE>;
-}
-
-// The kernel for rows of Z cells: a compile-time instance for rows of
-// 32..512 cells in powers of two (with its STALL form), else the runtime-row
-// instance whose thread bound covers Z / 2 (no STALL form: nullptr).
-template <bool STALL>
-static const void* pick_stream(int Z, int Y, bool ch, bool unit)
-{
-    switch (Z) {
-    case 32: return pick_mu<32, 32, 1, STALL, true>(ch, unit);
-    case 64: return pick_mu<64, 32, 2, STALL, true>(ch, unit);
-    case 128: return pick_mu<128, 64, 2, STALL, true>(ch, unit);
-    case 256: return pick_mu<256, 128, 2, STALL, true>(ch, unit);
-    case 512: return pick_mu<512, 256, 2, STALL, true>(ch, unit);
-    default: break;
-    }
-    if (STALL) return nullptr;
-    // Odd rows keep full-width shared rows (WIDE: every shared offset in the
-    // plane loop an immediate; 243^3 46.5 -> 42.9 us per step, 163^3 20.9 ->
-    // 18.2).  Rows of a multiple of 4 cells, and of 2 mod 4 cells on even Y,
-    // are bulk-copied as whole strips, which needs them contiguous in shared
-    // memory (one bulk copy per full-width row measured slower: 208^3 25.7 ->
-    // 29.9 us); for 2 mod 4 cells every piece then starts on an even row (R
-    // is even, and so is Y) and spans an even number of rows.
-    const int T = ch3_threads(Z, 2);
-    if (Z % 2) return T <= 128 ? pick_mu<0, 128, 2, false, false, true, true>(ch, unit)
-                               : pick_mu<0, 256, 2, false, false, true, true>(ch, unit);
-    const bool bulk = Z % 4 == 0 || (Y % 2 == 0 && kStreamR % 2 == 0);
-    if (T <= 128) return bulk ? pick_mu<0, 128, 2, false, true>(ch, unit) : pick_mu<0, 128, 2, false, false>(ch, unit);
-    return bulk ? pick_mu<0, 256, 2, false, true>(ch, unit) : pick_mu<0, 256, 2, false, false>(ch, unit);
-}
-
-// The shared row stride of the instance pick_stream chooses.
-static int stream_zs(int Z)
-{
-    if (Z % 2 == 0) return Z;
-    return ch3_threads(Z, 2) <= 128 ? 256 : 512;
+        return unit ? (const void*)&ch3_stream_f32<kStreamR, Z, MMSP_GPU_CH, true, STALL>
+                    : (const void*)&ch3_stream_f32<kStreamR, Z, MMSP_GPU_CH, false, STALL>;
+    return unit ? (const void*)&ch3_stream_f32<kStreamR, Z, MMSP_GPU_CH_POLY, true, STALL>
+                : (const void*)&ch3_stream_f32<kStreamR, Z, MMSP_GPU_CH_POLY, false, STALL>;
 }
 
 cudaError_t plan_ch3_stream(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
 {
     const Coeffs c = make_coeffs(d);
-    const int V = cells_per_thread(g.Z);
-    const int threads = ch3_threads(g.Z, V);
-    p->fn = pick_stream<false>(g.Z, g.Y, d.model == MMSP_GPU_CH, c.unit_w);
-    p->fn2 = pick_stream<true>(g.Z, g.Y, d.model == MMSP_GPU_CH, c.unit_w);   // the failure-detection test's form
-    p->smem = ch3_smem(kStreamR, g.Z, V, stream_zs(g.Z));
+    const bool ch = d.model == MMSP_GPU_CH;
+    const int threads = g.Z / 2;
+    p->fn = g.Z == 64 ? pick_stream<64, false>(ch, c.unit_w) : pick_stream<256, false>(ch, c.unit_w);
+    p->fn2 = g.Z == 64 ? pick_stream<64, true>(ch, c.unit_w) : pick_stream<256, true>(ch, c.unit_w);   // the test's form
+    p->smem = ch3_smem(kStreamR, g.Z);
     p->block = dim3(threads, 1, 1);
     cudaError_t e = ensure_smem(p->fn, p->smem);
-    if (e == cudaSuccess && p->fn2) e = ensure_smem(p->fn2, p->smem);
+    if (e == cudaSuccess) e = ensure_smem(p->fn2, p->smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->fn, threads, p->smem);
@@ -487,9 +348,9 @@ cudaError_t launch_ch3_stream(const StepPlan& p, const Geom& g, const Coeffs& c,
                               int* err, cudaStream_t s)
 {
     F32Coef q = f32coef(c);
-    int planes = p.planes;
-    void* args[] = {(void*)&in, (void*)&out, (void*)&g, (void*)&q, (void*)&planes, (void*)&err};
-    return cudaLaunchKernel(p.fn2 && take_stall() ? p.fn2 : p.fn, p.grid, p.block, args, p.smem, s);
+    int planes = p.planes, mirror = 0;
+    void* args[] = {(void*)&in, (void*)&out, (void*)&g, (void*)&q, (void*)&planes, (void*)&mirror, (void*)&err};
+    return cudaLaunchKernel(take_stall() ? p.fn2 : p.fn, p.grid, p.block, args, p.smem, s);
 }
 
 }  // namespace pf

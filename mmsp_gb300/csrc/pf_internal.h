@@ -83,6 +83,7 @@ struct StepPlan {
     int planes;        // planes of axis X per block (3D streaming)
     int fields;
     int kind;          // 0: the only kernel of its models' plan (CH tile, AC columns), 1: FP32 3D CH streaming,
+                       // 2: FP32 3D CH on warp windows of any rows,
                        // 3: FP32 CH rows of any length, 4: Ostwald ripening (two kernels),
                        // 5: convex splitting, 6: FP64 CH in two passes through a work grid,
                        // 8: FP32 3D Ostwald ripening streaming (one kernel)
@@ -94,11 +95,17 @@ struct StepPlan {
 cudaError_t plan_ch(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 cudaError_t plan_ac(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 
-// FP32 3D Cahn-Hilliard on whole rows (pf_ch3_stream.cu).
+// FP32 3D Cahn-Hilliard on rows of 256 cells, states above L2 (pf_ch3_stream.cu).
 bool ch3_stream_eligible(const mmsp_gpu_desc& d, const Geom& g);
 cudaError_t plan_ch3_stream(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 cudaError_t launch_ch3_stream(const StepPlan& p, const Geom& g, const Coeffs& c, const void* in, void* out,
                               int* err, cudaStream_t s);
+
+// FP32 3D Cahn-Hilliard on rows of any length (pf_ch3_flat.cu).
+bool ch3_flat_eligible(const mmsp_gpu_desc& d, const Geom& g);
+cudaError_t plan_ch3_flat(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
+cudaError_t launch_ch3_flat(const StepPlan& p, const Geom& g, const Coeffs& c, const void* in, void* out,
+                            cudaStream_t s);
 
 // FP64 2D/3D Cahn-Hilliard in two passes, mu into `work` (cells values),
 // then the update (pf_ch64.cu).  Needs the work grid, so only handles use it.
