@@ -291,7 +291,7 @@ static int take_stall()
 
 // Rows of 256 cells whose two states fill L2 or do not fit it: there the
 // ring's bulk copies keep more of HBM and L2 busy than the loads of
-// pf_ch3_flat.cu.  us per step, here / there: 256^3 (128 MB) 24.9 / 28.7,
+// pf_ch3_flat.cu.  us per step, here / there: 256^3 (128 MB) 24.6 / 28.7,
 // 512x256x256 45.0 / 52.5, 200x256x256 (100 MB) 20.5 / 23.9, 160x256x256 (80
 // MB) 17.2 / 18.2; 128x256x256 (64 MB) 14.9 / 14.2.  Every other row length is
 // faster there.
@@ -348,7 +348,7 @@ cudaError_t launch_ch3_stream(const StepPlan& p, const Geom& g, const Coeffs& c,
                               int* err, cudaStream_t s)
 {
     F32Coef q = f32coef(c);
-    int planes = p.planes, mirror = 0;
+    int planes = p.planes, mirror = in > out;
     void* args[] = {(void*)&in, (void*)&out, (void*)&g, (void*)&q, (void*)&planes, (void*)&mirror, (void*)&err};
     return cudaLaunchKernel(take_stall() ? p.fn2 : p.fn, p.grid, p.block, args, p.smem, s);
 }
