@@ -250,8 +250,6 @@ static void release(mmsp_gpu_handle* h)
 {
     if (h->out) pf::output_release(h);   // waits for snapshots still being written
     if (h->graph) cudaGraphExecDestroy(h->graph);
-    for (int p = 0; p < 2; p++)
-        if (h->cs_graph[p]) cudaGraphExecDestroy(h->cs_graph[p]);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->external) return;   // the caller's block and stream
@@ -629,25 +627,19 @@ static int build_graph(mmsp_gpu_handle* h)
 // (cahn-hilliard.cpp:311-388); then the guess becomes the state.
 static const unsigned kCsMaxIter = 10000;    // max_iter, cahn-hilliard.cpp:55
 static const unsigned kCsResidualStep = 5;   // residual_step, cahn-hilliard.cpp:54
-// A step is one CUDA graph per state buffer (pf_convex.cu,
-// build_convex_step_graph): its conditional `while` nodes run the checked
-// iterations and decide on the device, so a call queues one graph launch per
-// step and reads the loop state back once at the end.  The loop state lives
-// in the handle's status block.
+// A step is one cooperative launch (pf_convex.cu) that runs the whole solve
+// and decides on the device, so a call queues one launch per step and reads
+// the solve's outcome, which lives in the handle's status block, back once at
+// the end.
 static pf::CsLoop* convex_loop(mmsp_gpu_handle* h) { return reinterpret_cast<pf::CsLoop*>(h->flags + 16); }
 
 static int convex_steps(mmsp_gpu_handle* h, int steps)
 {
     cudaError_t e;
-    for (int p = 0; p < 2; p++)
-        if (!h->cs_graph[p] &&
-            (e = pf::build_convex_step_graph(h->d, h->g, h->c, h->buf[p], h->buf[p ^ 1], h->partials, convex_loop(h),
-                                             kCsMaxIter, kCsResidualStep, &h->cs_graph[p])) != cudaSuccess) {
-            h->cs_graph[p] = nullptr;
-            return cuda_fail(h, e, "convex step graph");
-        }
     for (int k = 0; k < steps; k++) {
-        if ((e = cudaGraphLaunch(h->cs_graph[h->cur], h->stream)) != cudaSuccess) return cuda_fail(h, e, "convex step");
+        e = pf::launch_convex_step(h->g, h->c, h->buf[h->cur], h->buf[h->cur ^ 1], h->partials, convex_loop(h),
+                                   h->flags, kCsMaxIter, kCsResidualStep, h->stream);
+        if (e != cudaSuccess) return cuda_fail(h, e, "convex step");
         h->cur ^= 1;   // swap(oldGrid, newGrid), cahn-hilliard.cpp:409
     }
     pf::CsLoop L;

@@ -47,7 +47,6 @@ struct mmsp_gpu_handle {
     cudaGraphExec_t graph;
     pf::OutputState* out;    // snapshot writer (mmsp_gpu_output), created on first use
     unsigned last_iters;     // MMSP_GPU_CH_CONVEX: solver iterations of the last step
-    cudaGraphExec_t cs_graph[2];   // MMSP_GPU_CH_CONVEX: one step (the solve's whole loop), per buf[cur]
     // 2D FP32 Cahn-Hilliard: blocks of pf::kTbAnyDepth steps per launch of the
     // temporally blocked kernel (its instance, tile list and work counters in `work`)
     bool tb;

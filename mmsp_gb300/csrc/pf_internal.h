@@ -148,29 +148,20 @@ cudaError_t plan_ost3_stream(const mmsp_gpu_desc& d, const Geom& g, const Coeffs
 cudaError_t launch_ost3_stream(const StepPlan& p, const Geom& g, const OstConst& o, const Coeffs& c,
                                const void* in, void* out, int* err, cudaStream_t s);
 
-// Convex-splitting Cahn-Hilliard (pf_convex.cu).  One red-black sweep
-// (color 1, then color 0 as the example orders them) of the guess `nw`
-// given the old state; and the residual reduction into partials
-// (result[0..1] = residual sum, norm of B, as launch_reduce leaves them).
-cudaError_t launch_convex_sweeps(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* old,
-                                 void* nw, cudaStream_t s);
-cudaError_t launch_convex_residual(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* old,
-                                   const void* nw, double* partials, cudaStream_t s);
-// The iteration loop of one convex-splitting step in device memory: the
-// iteration count and residual of the running solve, the count of the last
-// finished one, and a flag set when a solve reached max_iter.
+// Convex-splitting Cahn-Hilliard (pf_convex.cu).  What a step's solve leaves
+// in device memory: the last residual and iteration count, and a flag set
+// when it reached max_iter.
 struct CsLoop {
     double residual;
-    unsigned iter, last_iters;
-    int hit_max, pad;
+    unsigned last_iters;
+    int hit_max;
 };
-// One step as a CUDA graph (old -> guess nw): single iterations checked
-// while iter < first_checks, then chunks of first_checks iterations checked
-// at their ends, while the residual is above the tolerance and iter <
-// max_iter; conditional `while` nodes decide on the device.
-cudaError_t build_convex_step_graph(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* old, void* nw,
-                                    double* partials, CsLoop* L, unsigned max_iter, unsigned first_checks,
-                                    cudaGraphExec_t* exec);
+// One step (old -> guess nw) as one cooperative launch: red-black sweeps until
+// the residual, checked after iterations 1 .. first_checks-1 and every
+// first_checks-th, is at most the tolerance, or max_iter is reached; err is set
+// when a wait of its grid barrier runs out.
+cudaError_t launch_convex_step(const Geom& g, const Coeffs& c, const void* old, void* nw, double* partials, CsLoop* L,
+                               int* err, unsigned max_iter, unsigned first_checks, cudaStream_t s);
 
 // Sparse phase-field grain growth (pf_sparse.cu).  A state buffer holds
 // count[cells] int32 at 0, index[K][cells] int32 at idx_off and
