@@ -1,6 +1,7 @@
 // pf_aux.cu -- geometry/coefficients, FP64 compensated reductions, layout transposes.
 #include <math.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 
@@ -121,26 +122,34 @@ Coeffs make_coeffs(const mmsp_gpu_desc& d)
 // ---------------------------------------------------------------------------
 // Reductions.  Neumaier's compensated sum per thread, combined pairwise with
 // the same rule across the warp (shuffles), the block (shared memory) and
-// finally across blocks by one thread in block order, so the result depends
-// only on the data and the fixed launch shape.
+// finally across blocks, so the result depends only on the data and the
+// launch shape, which the grid fixes.
 
 struct NS {
     double s, c;
 };
 
-static __device__ __forceinline__ void nadd(NS& a, double x)
+// The larger of the two is told by its exponent and leading bits, on the
+// integer pipe: the error term is exact when its exponent is not the smaller.
+static __device__ __forceinline__ void nadd(const Ar<double>& A, NS& a, double x)
 {
-    double t = a.s + x;
-    if (fabs(a.s) >= fabs(x)) a.c += (a.s - t) + x;
-    else a.c += (x - t) + a.s;
+    const double t = A.add(a.s, x);
+    const bool sum_first = (__double2hiint(a.s) & 0x7fffffff) >= (__double2hiint(x) & 0x7fffffff);
+    const double big = sum_first ? a.s : x, small = sum_first ? x : a.s;
+    a.c = A.add(a.c, A.add(A.sub(big, t), small));
     a.s = t;
 }
 
-static __device__ __forceinline__ NS ncombine(NS a, NS b)
+// The lanes' sums of a warp, in a fixed order, on lane 0.
+static __device__ __forceinline__ NS nwarp(const Ar<double>& A, NS v)
 {
-    nadd(a, b.s);
-    a.c += b.c;
-    return a;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const NS o{__shfl_down_sync(0xffffffffu, v.s, off), __shfl_down_sync(0xffffffffu, v.c, off)};
+        nadd(A, v, o.s);
+        v.c = A.add(v.c, o.c);
+    }
+    return v;
 }
 
 struct RedArgs {
@@ -180,6 +189,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, Geom g, int N, RedArgs a,
                                                      double* __restrict__ partials)
 {
+    const Ar<double> A(g.dim);
     NS m{0.0, 0.0}, e{0.0, 0.0};
     const bool ch = a.model == MMSP_GPU_CH || a.model == MMSP_GPU_CH_POLY;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < g.cells;
@@ -198,8 +208,8 @@ __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, G
                 double c2 = C * C;
                 f = -0.5 * a.r * c2 + 0.25 * a.u * c2 * c2;
             }
-            nadd(e, f + 0.5 * a.kappa * gsq(st, g, a, x, y, z));
-            nadd(m, C);
+            nadd(A, e, f + 0.5 * a.kappa * gsq(st, g, a, x, y, z));
+            nadd(A, m, C);
         } else if (a.model == MMSP_GPU_CH_CONVEX) {
             // reportEnergy of the example (cahn-hilliard.cpp:172-200): energy_density(C)
             // + K/2 |grad C|^2 and the mass of C (field 1, the chemical potential, is not summed)
@@ -208,8 +218,8 @@ __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, G
             const double d0 = C - q.C0, da = C - q.Ca, db = C - q.Cb;
             const double f = -0.5 * q.A * d0 * d0 + 0.25 * q.B * d0 * d0 * d0 * d0 + 0.25 * q.Ca * da * da * da * da +
                              0.25 * q.Cb * db * db * db * db;
-            nadd(e, f + 0.5 * q.K * gsq(st, g, a, x, y, z));
-            nadd(m, C);
+            nadd(A, e, f + 0.5 * q.K * gsq(st, g, a, x, y, z));
+            nadd(A, m, C);
         } else if (a.model == MMSP_GPU_OSTWALD) {
             // f = -A/2 (C-Cm)^2 + B/4 (C-Cm)^4 + Da/4 (C-Ca)^4 + Db/4 (C-Cb)^4 - g/2 (C-Ca)^2 sum e^2
             //     + delta/4 sum e^4 + eps/2 sum_{i<j} e_i^2 e_j^2 + kappa/2 sum over all fields |grad|^2,
@@ -218,7 +228,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, G
             const double C = (double)st[i];
             const double dm = C - o.Cm, da = C - o.Ca, db = C - o.Cb;
             double grad = gsq(st, g, a, x, y, z), sq = 0.0, quart = 0.0, pair = 0.0;
-            nadd(m, C);
+            nadd(A, m, C);
             for (int j = 1; j < N; j++) {
                 const T* f = st + (long long)j * g.cells;
                 const double p = (double)f[i];
@@ -227,10 +237,10 @@ __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, G
                 pair += p2 * sq;
                 sq += p2;
                 grad += gsq(f, g, a, x, y, z);
-                nadd(m, p);
+                nadd(A, m, p);
             }
             const double dm2 = dm * dm, da2 = da * da, db2 = db * db;
-            nadd(e, -0.5 * o.A * dm2 + 0.25 * o.B * dm2 * dm2 + 0.25 * o.Da * da2 * da2 + 0.25 * o.Db * db2 * db2 -
+            nadd(A, e, -0.5 * o.A * dm2 + 0.25 * o.B * dm2 * dm2 + 0.25 * o.Da * da2 * da2 + 0.25 * o.Db * db2 * db2 -
                         0.5 * o.g * da2 * sq + 0.25 * o.delta * quart + 0.5 * o.eps * pair + 0.5 * o.kappa * grad);
         } else {
             double bulk = 0.0, pair = 0.0, grad = 0.0, sq = 0.0;
@@ -243,62 +253,47 @@ __global__ void __launch_bounds__(256) reduce_kernel(const T* __restrict__ st, G
                 pair += p2 * sq;
                 sq += p2;
                 grad += gsq(f, g, a, x, y, z);
-                nadd(m, p);
+                nadd(A, m, p);
             }
-            nadd(e, bulk + a.gamma * pair + 0.5 * a.kappa * grad);
+            nadd(A, e, bulk + a.gamma * pair + 0.5 * a.kappa * grad);
         }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        NS mo{__shfl_down_sync(0xffffffffu, m.s, off), __shfl_down_sync(0xffffffffu, m.c, off)};
-        NS eo{__shfl_down_sync(0xffffffffu, e.s, off), __shfl_down_sync(0xffffffffu, e.c, off)};
-        m = ncombine(m, mo);
-        e = ncombine(e, eo);
-    }
-    __shared__ double sh[8][4];
+    m = nwarp(A, m);
+    e = nwarp(A, e);
+    __shared__ NS sh[8][2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
-        sh[warp][0] = m.s;
-        sh[warp][1] = m.c;
-        sh[warp][2] = e.s;
-        sh[warp][3] = e.c;
+        sh[warp][0] = m;
+        sh[warp][1] = e;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        NS bm{0.0, 0.0}, be{0.0, 0.0};
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-            bm = ncombine(bm, NS{sh[w][0], sh[w][1]});
-            be = ncombine(be, NS{sh[w][2], sh[w][3]});
+    if (warp == 0) {
+        m = nwarp(A, lane < 8 ? sh[lane][0] : NS{0.0, 0.0});
+        e = nwarp(A, lane < 8 ? sh[lane][1] : NS{0.0, 0.0});
+        if (lane == 0) {
+            partials[blockIdx.x * 4 + 0] = m.s;
+            partials[blockIdx.x * 4 + 1] = m.c;
+            partials[blockIdx.x * 4 + 2] = e.s;
+            partials[blockIdx.x * 4 + 3] = e.c;
         }
-        partials[blockIdx.x * 4 + 0] = bm.s;
-        partials[blockIdx.x * 4 + 1] = bm.c;
-        partials[blockIdx.x * 4 + 2] = be.s;
-        partials[blockIdx.x * 4 + 3] = be.c;
     }
 }
 
-// One warp: lane l combines partials l, l+32, ... (its loads run in
-// parallel with the other lanes'), then lane 0 combines the 32 lane sums in
-// lane order.  The assignment is fixed, so the result is deterministic.
-__global__ void reduce_final(double* partials, int nblocks, double dV)
+// Two warps, one for the mass and one for the energy: lane l adds partials l,
+// l+32, ..., then the lanes' sums are added.  The order is fixed, so the result
+// is deterministic.  (Adding the 32 lane sums one after the other took 27 us:
+// every addition waits for the one before.)
+__global__ void __launch_bounds__(64) reduce_final(double* partials, int nblocks, double dV, int dim)
 {
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    NS m{0.0, 0.0}, e{0.0, 0.0};
+    const Ar<double> A(dim);
+    const int lane = threadIdx.x & 31, which = threadIdx.x >> 5;
+    NS v{0.0, 0.0};
     for (int b = lane; b < nblocks; b += 32) {
-        m = ncombine(m, NS{partials[b * 4 + 0], partials[b * 4 + 1]});
-        e = ncombine(e, NS{partials[b * 4 + 2], partials[b * 4 + 3]});
+        nadd(A, v, partials[b * 4 + 2 * which]);
+        v.c = A.add(v.c, partials[b * 4 + 2 * which + 1]);
     }
-    NS tm{0.0, 0.0}, te{0.0, 0.0};
-    for (int w = 0; w < 32; w++) {
-        const NS om{__shfl_sync(0xffffffffu, m.s, w), __shfl_sync(0xffffffffu, m.c, w)};
-        const NS oe{__shfl_sync(0xffffffffu, e.s, w), __shfl_sync(0xffffffffu, e.c, w)};
-        tm = ncombine(tm, om);
-        te = ncombine(te, oe);
-    }
-    if (lane == 0) {
-        partials[nblocks * 4 + 0] = dV * (tm.s + tm.c);
-        partials[nblocks * 4 + 1] = dV * (te.s + te.c);
-    }
+    v = nwarp(A, v);
+    if (lane == 0) partials[kReduceBlocks * 4 + which] = dV * (v.s + v.c);
 }
 
 cudaError_t launch_reduce(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c,
@@ -316,13 +311,15 @@ cudaError_t launch_reduce(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c
     a.cs = c.cs;
     int N = d.fields;
     if (gg) a.kappa = 2.0;   // graingrowth.cpp:105, zener.cpp:135: lap enters as 2*lap
+    // no more blocks than a small grid fills (the count depends on the grid alone)
+    const int blocks = (int)std::min((long long)kReduceBlocks, (g.cells + 255) / 256);
     if (d.dtype == MMSP_GPU_F64)
-        reduce_kernel<double><<<kReduceBlocks, 256, 0, s>>>((const double*)state, g, N, a, partials);
+        reduce_kernel<double><<<blocks, 256, 0, s>>>((const double*)state, g, N, a, partials);
     else
-        reduce_kernel<float><<<kReduceBlocks, 256, 0, s>>>((const float*)state, g, N, a, partials);
+        reduce_kernel<float><<<blocks, 256, 0, s>>>((const float*)state, g, N, a, partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    reduce_final<<<1, 32, 0, s>>>(partials, kReduceBlocks, c.dV);
+    reduce_final<<<1, 64, 0, s>>>(partials, blocks, c.dV, g.dim);
     return cudaGetLastError();
 }
 

@@ -180,8 +180,9 @@ cudaError_t launch_sparse_unpack(const void* state, void* staging, long long cel
 
 // Reductions: partial sums of (mass, energy) per block into `partials`
 // (4 doubles per block: mass sum, mass compensation, energy sum, energy
-// compensation), then a single-block pass into result[0..1] (mass, energy).
-// The block count is fixed (kReduceBlocks), so results do not depend on timing.
+// compensation), then a single-block pass into the two doubles behind
+// kReduceBlocks blocks' partials (mass, energy).  The block count depends on
+// the grid alone, so results do not depend on timing.
 constexpr int kReduceBlocks = 304;
 constexpr size_t kPartialsBytes = sizeof(double) * 4 * (kReduceBlocks + 1);
 cudaError_t launch_reduce(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c,
