@@ -320,6 +320,7 @@ int pf::create_in(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc, void* block,
 
 static int make_plan(mmsp_gpu_handle* h)
 {
+    h->multi = pf::plan_ch64_steps(h->d, h->g, &h->ch64s);
     if (h->d.model == MMSP_GPU_CH_CONVEX) {   // kernels are launched directly (pf_convex.cu)
         h->plan.kind = 5;
         h->plan.ok = true;
@@ -657,6 +658,11 @@ static int convex_steps(mmsp_gpu_handle* h, int steps)
     return MMSP_GPU_OK;
 }
 
+// Steps per launch of the small-grid kernel: a launch stays near a millisecond.
+static const int kMultiSteps = 256;
+// Its barrier word, in the handle's status block.
+static unsigned* multi_word(mmsp_gpu_handle* h) { return reinterpret_cast<unsigned*>(h->flags + 32); }
+
 extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
 {
     if (!h || steps < 0) return MMSP_GPU_EINVAL;
@@ -670,7 +676,17 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
         if (e != cudaSuccess) return cuda_fail(h, e, "sparse newGrid");
     }
     int left = steps;
-    if (h->d.model == MMSP_GPU_CH_CONVEX) {
+    if (h->multi) {
+        while (left > 0) {
+            const int n = std::min(left, kMultiSteps);
+            e = pf::launch_ch64_steps(h->ch64s, h->d, h->g, h->c, h->buf[h->cur], h->buf[h->cur ^ 1], n, multi_word(h),
+                                      h->multi_base, h->flags, h->stream);
+            if (e != cudaSuccess) return cuda_fail(h, e, "steps");
+            h->multi_base += (unsigned)(n - 1) * (unsigned)h->ch64s.blocks;
+            h->cur ^= n & 1;
+            left -= n;
+        }
+    } else if (h->d.model == MMSP_GPU_CH_CONVEX) {
         int rc = convex_steps(h, steps);
         if (rc) return rc;
         left = 0;
@@ -728,6 +744,10 @@ static int check_flags(mmsp_gpu_handle* h)
     if (e != cudaSuccess) return cuda_fail(h, e, "flags");
     if (f[0] || f[1]) {
         cudaMemset(h->flags, 0, sizeof(f));
+        if (h->multi) {   // a launch that left early leaves its barrier word anywhere
+            cudaMemset(multi_word(h), 0, sizeof(unsigned));
+            h->multi_base = 0;
+        }
         if (f[0]) return fail(h, MMSP_GPU_ETIMEDOUT, "%s", "a step kernel's bounded wait ran out; the state is invalid");
         return fail(h, MMSP_GPU_EOVERFLOW, "%s", "a sparse cell's list outgrew its slots (desc.fields); "
                                                   "the state is invalid");

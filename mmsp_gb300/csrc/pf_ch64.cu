@@ -26,6 +26,9 @@
 // the integer pipe (pf_device.cuh), and every decision about parameters
 // (unit weights, kappa == 1, noise) is a template argument, so no FP64
 // compare runs per cell.
+#include <algorithm>
+
+#include "pf_async.cuh"
 #include "pf_device.cuh"
 #include "pf_internal.h"
 
@@ -174,6 +177,141 @@ ch64_update(const double* __restrict__ cin, const double* __restrict__ mu, doubl
         cout[i] = o;
         a = b;
         b = n;
+    }
+}
+
+// Small 2D grids: many steps in one cooperative launch.  The two passes above
+// cost two launches a step, 1.6 us each however small the grid; here a block
+// per SM keeps its tile of c in shared memory, computes mu on the tile and one
+// cell around it, updates in place, and exchanges only the two outer cells of
+// each side with its neighbours, through the state buffers in turn, past a
+// grid barrier per step.  While the barrier's arrivals travel (1.3 us), a block
+// computes mu where it needs no neighbour.  (Announcing the outer cells before
+// the others are updated measured slower: 256^2 4.35 us per step, one more
+// phase to wait through.)  Each mu is computed with the
+// operations of ch64_mu, so the rim that two blocks both compute has the same
+// bits, and the states are those of the two passes.
+constexpr int kC64StepThreads = 512;
+
+struct C64Tiles {
+    int h, w, nz;   // rows and columns of a tile, tiles along Z
+};
+
+// Cell e of a frame two cells wide around an h x w interior: its row and column
+// in the (h+4) x (w+4) frame.
+static __device__ __forceinline__ void frame_cell(int e, int h, int w, int& r, int& c)
+{
+    if (e < 4 * (w + 4)) {
+        r = e / (w + 4);
+        c = e - r * (w + 4);
+        r = r < 2 ? r : h + r;
+    } else {
+        const int m = e - 4 * (w + 4);
+        r = 2 + (m >> 2);
+        c = (m & 3) < 2 ? (m & 3) : w + (m & 3);
+    }
+}
+
+template <int MODEL, bool UNIT, bool KONE, bool EXACT>
+__global__ void __launch_bounds__(kC64StepThreads)
+ch64_steps(double* s0, double* s1, Geom g, C64 q0, P<double> p0, C64Tiles tl, int steps, unsigned* count, unsigned base,
+           int* err)
+{
+    const Ar<double> A(g.dim);
+    const C64 q = held(A, q0);
+    const P<double> p = held(A, p0);
+    extern __shared__ double tile_sm[];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x;
+    const int y0 = (int)(blockIdx.x / tl.nz) * tl.h, z0 = (int)(blockIdx.x % tl.nz) * tl.w;
+    const int h = min(tl.h, g.Y - y0), w = min(tl.w, g.Z - z0);
+    const int CW = tl.w + 4, MW = tl.w + 2;
+    double* C = tile_sm;                       // c with two cells around: [h+4][CW]
+    double* M = C + (tl.h + 4) * CW;           // mu with one cell around: [h+2][MW]
+    auto where = [&](int r, int c) {           // cell (r, c) of C in a state buffer
+        return (long long)wrapi(y0 - 2 + r, g.Y) * g.Z + wrapi(z0 - 2 + c, g.Z);
+    };
+    auto mu_at = [&](int r, int c) {           // mu of cell (r, c) of M
+        const double* k = C + (r + 1) * CW + c + 1;
+        M[r * MW + c] = mu_cell<2, MODEL, UNIT, KONE, EXACT>(A, k[0], 0.0, 0.0, k[CW], k[-CW], k[1], k[-1], q, p);
+    };
+    // mu without neighbours' cells: the (h-2) x (w-2) cells two inside M
+    const int ih = h - 2, iw = w - 2;
+    const bool inner = ih > 0 && iw > 0;
+    const int inner_n = inner ? ih * iw : 0, rim_n = inner ? (h + 2) * (w + 2) - inner_n : 0;
+
+    for (int e = tid; e < (h + 4) * (w + 4); e += kC64StepThreads) {
+        const int r = e / (w + 4), c = e - r * (w + 4);
+        C[r * CW + c] = __ldcg(s0 + where(r, c));
+    }
+    __syncthreads();
+    for (int e = tid; e < inner_n; e += kC64StepThreads) {
+        const int r = e / iw;
+        mu_at(r + 2, e - r * iw + 2);
+    }
+    for (int s = 0; s < steps; s++) {
+        // the rest of mu
+        if (inner) {
+            for (int e = tid; e < rim_n; e += kC64StepThreads) {
+                int r, c;
+                frame_cell(e, ih, iw, r, c);
+                mu_at(r, c);
+            }
+        } else {
+            for (int e = tid; e < (h + 2) * (w + 2); e += kC64StepThreads) {
+                const int r = e / (w + 2);
+                mu_at(r, e - r * (w + 2));
+            }
+        }
+        __syncthreads();
+        // the update in place; a cell that a neighbour will read, or any at the end, to the next state buffer
+        double* dst = s & 1 ? s0 : s1;
+        const bool last = s + 1 == steps;
+        for (int e = tid; e < h * w; e += kC64StepThreads) {
+            const int r = e / w, c = e - r * w;
+            const double* m = M + (r + 1) * MW + c + 1;
+            double* k = C + (r + 2) * CW + c + 2;
+            double o;
+            if (EXACT) {
+                const double lap = lap_ref<double, UNIT, 2>(A, twice(m[0]), 0.0, 0.0, m[MW], m[-MW], m[1], m[-1], p.wx, p.wy, p.wz);
+                o = A.add(*k, A.mul(p.dtm, lap));
+            } else {
+                o = fma(q.dtm, nsum<2, UNIT>(A, 0.0, A.add(m[MW], m[-MW]), A.add(m[1], m[-1]), q), fma(q.upd0, m[0], *k));
+            }
+            *k = o;
+            if (last || r < 2 || r >= h - 2 || c < 2 || c >= w - 2) dst[(long long)(y0 + r) * g.Z + z0 + c] = o;
+        }
+        if (last) break;
+        // arrive, compute what needs no other block, wait
+        __syncthreads();
+        if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        for (int e = tid; e < inner_n; e += kC64StepThreads) {
+            const int r = e / iw;
+            mu_at(r + 2, e - r * iw + 2);
+        }
+        if (tid == 0) {
+            const unsigned target = base + (unsigned)(s + 1) * gridDim.x;
+            const uint64_t t0 = global_ns();
+            bool done = false;
+            for (unsigned spin = 0; !done; spin++) {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+                done = (int)(v - target) >= 0;
+                if (!done && (spin & 255u) == 255u && global_ns() - t0 > kWaitNs) break;
+            }
+            s_ok = done;
+        }
+        __syncthreads();
+        if (!s_ok) {   // the other blocks' waits run out too
+            if (tid == 0) atomicExch(err, 1);
+            return;
+        }
+        for (int e = tid; e < 4 * (w + 4) + 4 * h; e += kC64StepThreads) {
+            int r, c;
+            frame_cell(e, h, w, r, c);
+            C[r * CW + c] = __ldcg(dst + where(r, c));
+        }
+        __syncthreads();
     }
 }
 
@@ -387,6 +525,76 @@ cudaError_t launch_ch64(const StepPlan& p, const mmsp_gpu_desc& d, const Geom& g
     const void* mu = work;
     void* a2[] = {(void*)&in, (void*)&mu, (void*)&out, (void*)&g, (void*)&q, (void*)&pp, (void*)&planes};
     return cudaLaunchKernel(p.fn2, p.grid, p.block, a2, 0, s);
+}
+
+namespace {
+
+template <int MODEL, bool UNIT>
+const void* steps_fn_u(bool kone, bool exact)
+{
+    if (kone) return exact ? (const void*)&ch64_steps<MODEL, UNIT, true, true> : (const void*)&ch64_steps<MODEL, UNIT, true, false>;
+    return exact ? (const void*)&ch64_steps<MODEL, UNIT, false, true> : (const void*)&ch64_steps<MODEL, UNIT, false, false>;
+}
+
+template <int MODEL>
+const void* steps_fn(bool unit, bool kone, bool exact)
+{
+    return unit ? steps_fn_u<MODEL, true>(kone, exact) : steps_fn_u<MODEL, false>(kone, exact);
+}
+
+}  // namespace
+
+// us per step, two passes / here (256 steps a call): 64^2 3.6 / 3.1, 256^2 5.1 /
+// 4.0 (contracted 4.2 / 3.2), 400^2 7.9 / 7.1, 512^2 10.9 / 10.3, 640x600 14.2 /
+// 13.2; in calls of 20 steps, which the two passes launch one by one, 8.5 /
+// 3.5 at 64^2 and 18.7 / 13.8 at 640x600.  Above, the FP64 work of the tiles'
+// rims outweighs the launches.
+constexpr long long kC64StepsMost = 400LL << 10;
+
+bool plan_ch64_steps(const mmsp_gpu_desc& d, const Geom& g, Ch64Steps* p)
+{
+    if (d.dtype != MMSP_GPU_F64 || g.dim != 2 || noisy(d) || g.cells > kC64StepsMost ||
+        (d.model != MMSP_GPU_CH && d.model != MMSP_GPU_CH_POLY))
+        return false;
+    const Coeffs c = make_coeffs(d);
+    const bool exact = !(d.flags & MMSP_GPU_FLAG_CONTRACT), kone = c.kappa == 1.0;
+    p->fn = d.model == MMSP_GPU_CH ? steps_fn<MMSP_GPU_CH>(c.unit_w, kone, exact)
+                                   : steps_fn<MMSP_GPU_CH_POLY>(c.unit_w, kone, exact);
+    // tiles that leave an SM the least FP64 work: 10 operations per mu, 7 per update
+    const int sms = sm_count();
+    long long best = -1;
+    for (int nz = 1; nz <= std::min(sms, g.Z); nz++) {
+        const int ny = std::min(sms / nz, g.Y);
+        const int h = (g.Y + ny - 1) / ny, w = (g.Z + nz - 1) / nz;
+        const long long work = 10LL * (h + 2) * (w + 2) + 7LL * h * w;
+        if (best < 0 || work < best) {
+            best = work;
+            p->h = h;
+            p->w = w;
+        }
+    }
+    p->nz = (g.Z + p->w - 1) / p->w;
+    p->blocks = (g.Y + p->h - 1) / p->h * p->nz;
+    p->smem = sizeof(double) * ((size_t)(p->h + 4) * (p->w + 4) + (size_t)(p->h + 2) * (p->w + 2));
+    // one block per SM fits at 512 threads of at most 64 registers
+    if (p->smem > 200 * 1024) return false;
+    if (p->smem > 48 * 1024 && ensure_smem(p->fn, p->smem) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
+cudaError_t launch_ch64_steps(const Ch64Steps& p, const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, void* in,
+                              void* other, int steps, unsigned* count, unsigned base, int* err, cudaStream_t s)
+{
+    C64 q = c64_of(c, g.dim);
+    q.poly0 = (d.model == MMSP_GPU_CH ? 2.0 : c.neg_r) + c.kappa * q.w2;
+    P<double> pp = narrow<double>(c, g.dim);
+    C64Tiles tl{p.h, p.w, p.nz};
+    void* args[] = {(void*)&in, (void*)&other, (void*)&g, (void*)&q, (void*)&pp, (void*)&tl, (void*)&steps, (void*)&count,
+                    (void*)&base, (void*)&err};
+    return cudaLaunchCooperativeKernel(p.fn, dim3(p.blocks), dim3(kC64StepThreads), args, p.smem, s);
 }
 
 }  // namespace pf

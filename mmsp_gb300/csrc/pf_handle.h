@@ -47,6 +47,10 @@ struct mmsp_gpu_handle {
     cudaGraphExec_t graph;
     pf::OutputState* out;    // snapshot writer (mmsp_gpu_output), created on first use
     unsigned last_iters;     // MMSP_GPU_CH_CONVEX: solver iterations of the last step
+    // small 2D FP64 Cahn-Hilliard: many steps per cooperative launch; the value of its barrier word
+    bool multi;
+    pf::Ch64Steps ch64s;
+    unsigned multi_base;
     // 2D FP32 Cahn-Hilliard: blocks of pf::kTbAnyDepth steps per launch of the
     // temporally blocked kernel (its instance, tile list and work counters in `work`)
     bool tb;

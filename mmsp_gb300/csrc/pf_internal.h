@@ -114,6 +114,19 @@ cudaError_t plan_ch64(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 cudaError_t launch_ch64(const StepPlan& p, const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* in,
                         void* out, void* work, int* err, cudaStream_t s);
 
+// Many steps of a small 2D FP64 Cahn-Hilliard grid in one cooperative launch
+// (pf_ch64.cu), between the two state buffers in turn; false: the grid takes
+// the two passes.  `count` is a device word of the caller's that the launch's
+// steps-1 grid barriers raise by `blocks` each; `base` is its value before.
+struct Ch64Steps {
+    const void* fn;
+    int h, w, nz, blocks;   // tile rows and columns, tiles along Z, tiles
+    size_t smem;
+};
+bool plan_ch64_steps(const mmsp_gpu_desc& d, const Geom& g, Ch64Steps* p);
+cudaError_t launch_ch64_steps(const Ch64Steps& p, const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, void* in,
+                              void* other, int steps, unsigned* count, unsigned base, int* err, cudaStream_t s);
+
 // FP32 2D/3D Cahn-Hilliard for any row length up to 1024 (pf_rows.cu).
 bool ch_rows_eligible(const mmsp_gpu_desc& d, const Geom& g);
 cudaError_t plan_ch_rows(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
