@@ -578,7 +578,7 @@ bool plan_ch64_steps(const mmsp_gpu_desc& d, const Geom& g, Ch64Steps* p)
     p->smem = sizeof(double) * ((size_t)(p->h + 4) * (p->w + 4) + (size_t)(p->h + 2) * (p->w + 2));
     // one block per SM fits at 512 threads of at most 64 registers
     if (p->smem > 200 * 1024) return false;
-    if (p->smem > 48 * 1024 && ensure_smem(p->fn, p->smem) != cudaSuccess) {
+    if (p->smem > 40 * 1024 && ensure_smem(p->fn, p->smem) != cudaSuccess) {   // (48 KB with the static part)
         cudaGetLastError();
         return false;
     }
