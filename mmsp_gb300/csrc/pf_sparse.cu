@@ -16,8 +16,8 @@
 // sets the overflow word and leaves that item out (the host reports
 // MMSP_GPU_EOVERFLOW; the state is then invalid).
 //
-// One thread per cell.  The example's newGrid starts with empty cells and is
-// never cleared: after swap() the buffer written at step s holds the state of
+// The example's newGrid starts with empty cells and is never cleared:
+// after swap() the buffer written at step s holds the state of
 // step s-2, and set() keeps the items it does not overwrite.  The ping-pong
 // buffers do the same (the host clears the idle buffer's counts at the start
 // of each step call, as each update() call builds a fresh newGrid), so the
@@ -79,16 +79,14 @@ struct SpConst {
     P<double> p;     // dtm = dt for the update expression
 };
 
+// The padded coordinates' neighbours of one cell in the reference's axis order
+// (real axis 0 first), then the update of its lists, list by list in global
+// memory: any number of grains.
 template <int DIM, bool UNIT>
-__global__ void __launch_bounds__(128)
-sparse_gg_step(SpView in, SpView out, Geom g, SpConst q, int K, int* __restrict__ err)
+static __device__ __noinline__ void sparse_cell(SpView in, SpView out, Geom g, SpConst q, int K, long long c, int* err)
 {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= g.cells) return;
     const long long cells = g.cells;
     const Ar<double> A(g.dim);
-    // padded coordinates and the periodic face neighbours of the real axes,
-    // in the reference's axis order (real axis 0 first)
     const int x = (int)(c / g.YZ);
     const int r = (int)(c - (long long)x * g.YZ);
     const int y = r / g.Z;
@@ -173,6 +171,167 @@ sparse_gg_step(SpView in, SpView out, Geom g, SpConst q, int K, int* __restrict_
     if (ovf) atomicExch(err, 1);
 }
 
+// One thread per cell.  The neighbour lists are read once: the union is built
+// in shared memory, one column per thread, and beside each of its grains the
+// slots that the grain has in the cell's, the neighbours' and the destination
+// list, 6 bits each.  Every value is then one direct load, and the loads of a
+// grain are independent of each other.  A union of more than kSpUnion grains
+// goes through sparse_cell.
+//
+// Bound: the FP64 pipe (about 18 operations per cell and grain, and a warp
+// takes as many rounds as its busiest cell; 55% busy) and load latency.  us per
+// step, walking the lists in global memory for every value / here: 512x512
+// cells of 160 grains 78.5 / 55.1 (500 steps from one item per cell; 60 steps
+// 55.5 / 41.8), 2048x2048 of 32 grains 201 / 154, 48^3 of 12 grains 100 / 58.
+// (A dense table of a tile's grains in shared memory, behind a hashed
+// dictionary, took 65, 64, 229 and 82: its set-up costs more than the walks.)
+// 64-thread blocks of at most 64 registers: with 128 threads 60.9, with 72
+// registers 58.6.
+constexpr int kSpThreads = 64;
+constexpr int kSpUnion = 16;
+constexpr int kSpBatch = 4;   // items of a list that are loaded at once
+
+template <int DIM, bool UNIT>
+__global__ void __launch_bounds__(kSpThreads, 16)
+sparse_gg_step(SpView in, SpView out, Geom g, SpConst q0, int K, int* __restrict__ err)
+{
+    __shared__ int s_key[kSpUnion][kSpThreads];
+    __shared__ unsigned long long s_pos[kSpUnion][kSpThreads];   // slot + 1 in list l at bit 6*l, 0: not there
+    const int tid = threadIdx.x;
+    const long long c = (long long)blockIdx.x * kSpThreads + tid;
+    if (c >= g.cells) return;   // no barrier in this kernel
+    const long long cells = g.cells;
+    // padded coordinates and the periodic face neighbours of the real axes,
+    // in the reference's axis order (real axis 0 first); list 0 is the cell's
+    // own, 1 + 2 ra and 2 + 2 ra the low and high neighbour's on axis ra, 7 the
+    // destination's
+    const int x = (int)(c / g.YZ);
+    const int r = (int)(c - (long long)x * g.YZ);
+    const int y = r / g.Z;
+    const int z = r - y * g.Z;
+    long long nb[1 + 2 * DIM];
+    nb[0] = c;
+    nb[2 * DIM - 1] = c + (z == 0 ? g.Z - 1 : -1);
+    nb[2 * DIM] = c + (z + 1 == g.Z ? -z : 1);
+    if constexpr (DIM >= 2) {
+        nb[2 * DIM - 3] = c + (long long)(y == 0 ? g.Y - 1 : -1) * g.Z;
+        nb[2 * DIM - 2] = c + (long long)(y + 1 == g.Y ? -y : 1) * g.Z;
+    }
+    if constexpr (DIM == 3) {
+        nb[1] = c + (long long)(x == 0 ? g.X - 1 : -1) * g.YZ;
+        nb[2] = c + (long long)(x + 1 == g.X ? -x : 1) * g.YZ;
+    }
+    int n[1 + 2 * DIM];
+#pragma unroll
+    for (int l = 0; l < 1 + 2 * DIM; l++) n[l] = __ldg(in.cnt + nb[l]);
+
+    int ns = 0;
+    // items of list l into the union (JOIN), or only their slots
+    auto read = [&](const int* idx, long long cell, int items, int l, bool join) {
+        for (int h0 = 0; h0 < items; h0 += kSpBatch) {
+            int key[kSpBatch];
+#pragma unroll
+            for (int k = 0; k < kSpBatch; k++) key[k] = h0 + k < items ? idx[(h0 + k) * cells + cell] : 0;
+#pragma unroll
+            for (int k = 0; k < kSpBatch; k++) {
+                if (h0 + k >= items) break;
+                int s = 0;
+                while (s < ns && s_key[s][tid] != key[k]) s++;
+                const unsigned long long slot = (unsigned long long)(h0 + k + 1) << (6 * l);
+                if (s < ns) {
+                    // (of a repeated index the first item counts)
+                    const unsigned long long have = s_pos[s][tid];
+                    if (!(have >> (6 * l) & 63)) s_pos[s][tid] = have | slot;
+                } else if (join) {
+                    if (ns < kSpUnion) {
+                        s_key[ns][tid] = key[k];
+                        s_pos[ns][tid] = slot;
+                    }
+                    if (ns <= kSpUnion) ns++;
+                    if (ns > kSpUnion) return;
+                }
+            }
+        }
+    };
+    // the example's visiting order: per axis the low neighbour, the cell itself, the high neighbour
+#pragma unroll
+    for (int ra = 0; ra < DIM; ra++) {
+        if (ns <= kSpUnion) read(in.idx, nb[1 + 2 * ra], n[1 + 2 * ra], 1 + 2 * ra, true);
+        if (ra == 0 && ns <= kSpUnion) read(in.idx, c, n[0], 0, true);
+        if (ns <= kSpUnion) read(in.idx, nb[2 + 2 * ra], n[2 + 2 * ra], 2 + 2 * ra, true);
+    }
+    if (ns > kSpUnion) {
+        sparse_cell<DIM, UNIT>(in, out, g, q0, K, c, err);
+        return;
+    }
+    if (ns < 2) {
+        // newGrid(n) = oldGrid(n): the whole list
+        out.cnt[c] = n[0];
+        for (int h = 0; h < n[0]; h++) {
+            out.idx[h * cells + c] = __ldg(in.idx + h * cells + c);
+            out.val[h * cells + c] = __ldg(in.val + h * cells + c);
+        }
+        return;
+    }
+    const Ar<double> A(g.dim);
+    const P<double> p = held(A, q0.p);
+    double sum = 0.0;
+    for (int h0 = 0; h0 < n[0]; h0 += kSpBatch) {
+        double v[kSpBatch];
+#pragma unroll
+        for (int k = 0; k < kSpBatch; k++) v[k] = h0 + k < n[0] ? __ldg(in.val + (h0 + k) * cells + c) : 0.0;
+#pragma unroll
+        for (int k = 0; k < kSpBatch; k++) {
+            if (h0 + k >= n[0]) break;
+            sum = A.add(sum, A.mul(v[k], v[k]));
+        }
+    }
+    // newGrid(n) as it stands: the state of two steps back
+    int dn = out.cnt[c];
+    read(out.idx, c, dn, 7, false);
+    bool ovf = false;
+    // the values of grain s in the cell's and the neighbours' lists
+    auto fetch = [&](int s, double (&f)[1 + 2 * DIM]) {
+        const unsigned long long pos = s_pos[s][tid];
+#pragma unroll
+        for (int l = 0; l < 1 + 2 * DIM; l++) {
+            const int slot = (int)(pos >> (6 * l)) & 63;
+            f[l] = slot ? __ldg(in.val + (slot - 1) * cells + nb[l]) : 0.0;
+        }
+    };
+    double next[1 + 2 * DIM];   // loaded one grain ahead
+    fetch(0, next);
+    for (int s = 0; s < ns; s++) {
+        double f[1 + 2 * DIM];
+#pragma unroll
+        for (int l = 0; l < 1 + 2 * DIM; l++) f[l] = next[l];
+        if (s + 1 < ns) fetch(s + 1, next);
+        const double phi = f[0], y2 = twice(phi);
+        double lap = 0.0;
+#pragma unroll
+        for (int ra = 0; ra < DIM; ra++) {
+            double t = A.add(A.sub(f[2 + 2 * ra], y2), f[1 + 2 * ra]);
+            if (!UNIT) t = A.mul(A.reg(q0.w[ra]), t);
+            lap = ra == 0 ? plus_zero(t) : A.add(lap, t);
+        }
+        const double v = ac_new<double, MMSP_GPU_GG>(A, phi, sum, lap, p);
+        if (v > q0.eps) {
+            int h = (int)(s_pos[s][tid] >> 42) & 63;
+            if (!h) {
+                if (dn == K) {
+                    ovf = true;
+                    continue;
+                }
+                out.idx[dn * cells + c] = s_key[s][tid];
+                h = ++dn;
+            }
+            out.val[(h - 1) * cells + c] = v;
+        }
+    }
+    out.cnt[c] = dn;
+    if (ovf) atomicExch(err, 1);
+}
+
 // Host cell-major slots (count[cells], index[cells*K], value[cells*K]) <->
 // the device's slot-major buffer, through a staging buffer that holds the
 // three host arrays at the offsets of sparse_layout.
@@ -202,7 +361,7 @@ __global__ void sparse_unpack(SpView d, int* __restrict__ hcnt, int* __restrict_
     }
 }
 
-static unsigned blocks_for(long long cells) { return (unsigned)((cells + 127) / 128); }
+static unsigned blocks_for(long long cells, int threads = 128) { return (unsigned)((cells + threads - 1) / threads); }
 
 cudaError_t launch_sparse_gg(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* in, void* out,
                              int* err, cudaStream_t s)
@@ -219,7 +378,7 @@ cudaError_t launch_sparse_gg(const mmsp_gpu_desc& d, const Geom& g, const Coeffs
     else fn = c.unit_w ? (const void*)&sparse_gg_step<1, true> : (const void*)&sparse_gg_step<1, false>;
     int* ovf = err + 1;
     void* args[] = {(void*)&vi, (void*)&vo, (void*)&g, (void*)&q, (void*)&K, (void*)&ovf};
-    return cudaLaunchKernel(fn, dim3(blocks_for(g.cells)), dim3(128), args, 0, s);
+    return cudaLaunchKernel(fn, dim3(blocks_for(g.cells, kSpThreads)), dim3(kSpThreads), args, 0, s);
 }
 
 cudaError_t launch_sparse_pack(const void* staging, void* state, long long cells, int K, cudaStream_t s)
