@@ -711,7 +711,7 @@ def batched(native, inputs, stream, reps, flush):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": profile_traffic("ch2_tb_f32_256grids" if info.temporal_depth > 1
                                                 else "ch2_batch_f32_256grids"),
-                     "kernel": ("ch2_tb_kernel<region %dx%d, KS=%d, CH, unit> (%d steps per launch)" % (
+                     "kernel": ("temporally blocked, CH, region %dx%d, KS=%d (%d steps per launch)" % (
                          info.tile_rows, info.tile_cols, info.temporal_depth, info.temporal_depth)
                                 if info.temporal_depth > 1 else "ch2_batch_kernel<float,CH>"),
                      "peak_source": peak_kind, "alg_bytes_per_step": cells * 8,

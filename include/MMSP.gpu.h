@@ -317,10 +317,11 @@ int mmsp_gpu_output_wait(mmsp_gpu_handle* h);
  * graph.  FP32 batches whose grids all join the persistent kernel can also
  * advance by temporal blocking: each launch loads tiles of every grid with a
  * halo of 2 cells per step into shared memory, takes 2, 4 or 8 steps there
- * and writes the tiles back, cutting HBM traffic per step by about that
- * factor for some redundant halo work.  The run of rows per work item and
- * the block size of the per-step kernel, and the tile region and steps per
- * launch of the blocked one (or none), are chosen by an autotuner on the
+ * and writes the tiles back, or streams strips of rows through four steps in
+ * registers, cutting HBM traffic per step by about that factor for some
+ * redundant halo work.  The run of rows per work item and
+ * the block size of the per-step kernel, and the tile region or strip and steps
+ * per launch of the blocked one (or none), are chosen by an autotuner on the
  * first step (or mmsp_gpu_batch_tune) and cached per batch shape, in memory
  * and, when the environment variable MMSP_GPU_TUNE_CACHE names a file, in
  * that JSON file.  The environment variable MMSP_GPU_BATCH_TILE="depth,shape"
@@ -343,8 +344,8 @@ typedef struct mmsp_gpu_batch_info {
     double tune_ms;         /* wall time spent autotuning */
     size_t device_bytes;    /* device memory the batch holds */
     int temporal_depth;     /* steps per launch of the persistent kernel: 1, or the autotuned depth of
-                               the temporally blocked kernel (shared-memory tiles, FP32) */
-    int tile_rows, tile_cols;   /* its tile region (halo included), 0 when not used */
+                               a temporally blocked kernel (shared-memory tiles, or strips, FP32) */
+    int tile_rows, tile_cols;   /* its tile or strip region (halo included), 0 when not used */
     int tiles;              /* its work items per launch */
 } mmsp_gpu_batch_info;
 

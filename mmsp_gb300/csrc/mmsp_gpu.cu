@@ -208,11 +208,17 @@ static bool two_pass_f64(const mmsp_gpu_desc* d)
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // 2D FP32 Cahn-Hilliard grids step in blocks of pf::kTbAnyDepth steps, each
-// one launch of the temporally blocked kernel of the batched form
-// (pf_batch.cu) over the grid's 64 x 128 regions: a quarter of the launches
-// and of the HBM traffic of one kernel per step.  The leftover steps of a
-// call (fewer than kTbAnyDepth) take the plan's per-step kernel, so a run
-// split into calls of multiples of kTbAnyDepth steps equals one call.
+// one launch of a temporally blocked kernel of the batched form (pf_batch.cu):
+// a quarter of the launches and of the HBM traffic of one kernel per step.  The
+// leftover steps of a call (fewer than kTbAnyDepth) take the plan's per-step
+// kernel, so a run split into calls of multiples of kTbAnyDepth steps equals
+// one call.  The strip kernel takes the grids of kStripMinRows rows and more,
+// the tile kernel (64 x 128 regions) those of fewer: the strips' lead of 19
+// rounds is a fixed price, the tile's work follows its rows.  us per step, tile
+// against strips: 8 rows of 64 cells 1.11 / 1.27, 12 rows of 128 1.27 / 1.33,
+// 16 rows of 128 1.30 / 1.33, 24 rows of 128 1.56 / 1.34, 64 of 64 1.87 / 1.33.
+static_assert(pf::kStripKS == pf::kTbAnyDepth, "one depth for both kernels");
+static const int kStripMinRows = 24;
 static bool tb_handle(const mmsp_gpu_desc* d)
 {
     return d->dtype == MMSP_GPU_F32 && d->dim == 2 && (d->model == MMSP_GPU_CH || d->model == MMSP_GPU_CH_POLY) &&
@@ -222,16 +228,22 @@ static bool tb_handle(const mmsp_gpu_desc* d)
 static int tb_tile_rows() { return pf::kTbShapes[0].ri - 4 * pf::kTbAnyDepth; }
 static int tb_tile_cols() { return pf::kTbCols - 4 * pf::kTbAnyDepth; }
 
+static bool tb_strips(const mmsp_gpu_desc* d) { return d->n[0] >= kStripMinRows; }
+
 static size_t tb_meta_bytes(const mmsp_gpu_desc* d)
 {
-    const long long tiles = (long long)((d->n[0] + tb_tile_rows() - 1) / tb_tile_rows()) *
-                            ((d->n[1] + tb_tile_cols() - 1) / tb_tile_cols());
-    return align256(sizeof(pf::BatchInst)) + align256(sizeof(pf::TbItem) * (size_t)tiles) + 256;
+    const int n0 = d->n[0], n1 = d->n[1];
+    const size_t inst = align256(sizeof(pf::BatchInst));
+    if (tb_strips(d))
+        return inst + align256(sizeof(pf::StripItem) * (size_t)pf::strip_windows(n0, n1, pf::strip_rows(n0, n1)));
+    const long long tiles = (long long)((n0 + tb_tile_rows() - 1) / tb_tile_rows()) *
+                            ((n1 + tb_tile_cols() - 1) / tb_tile_cols());
+    return inst + align256(sizeof(pf::TbItem) * (size_t)tiles) + 256;
 }
 
 static size_t work_bytes(const mmsp_gpu_desc* d)
 {
-    if (tb_handle(d)) return tb_meta_bytes(d);   // the blocked kernel's instance, tiles and counters
+    if (tb_handle(d)) return tb_meta_bytes(d);   // the blocked kernels' instance, list and counters
     if (d->model == MMSP_GPU_CH_CONVEX) return state_bytes(d);   // download staging (the guess stays put)
     if (d->model != MMSP_GPU_OSTWALD && !two_pass_f64(d)) return 0;
     return state_bytes(d) / (size_t)d->fields;
@@ -342,15 +354,16 @@ static int make_plan(mmsp_gpu_handle* h)
     return MMSP_GPU_OK;
 }
 
-// The blocked kernel's instance and tile list, in the handle's work buffer.
+// The blocked kernels' instance and list, in the handle's work buffer.
+// Queued on the handle's stream, ahead of its first launch, with no
+// synchronisation: a server request's stream may carry another request's
+// queued steps.  A copy from pageable memory has staged its source when the
+// call returns, so the host arrays may go out of scope.
 static int setup_tb(mmsp_gpu_handle* h)
 {
     if (!tb_handle(&h->d)) return MMSP_GPU_OK;
-    const int n0 = h->d.n[0], n1 = h->d.n[1], TX = tb_tile_rows(), TZ = tb_tile_cols();
-    std::vector<pf::TbItem> items;
-    for (int x0 = 0; x0 < n0; x0 += TX)
-        for (int z0 = 0; z0 < n1; z0 += TZ)
-            items.push_back(pf::TbItem{0, x0, z0, std::min(TX, n0 - x0), std::min(TZ, n1 - z0)});
+    const int n0 = h->d.n[0], n1 = h->d.n[1];
+    const bool aligned = n1 % 4 == 0;   // 16-byte row groups
     pf::BatchInst bi;
     memset(&bi, 0, sizeof(bi));
     bi.off = 0;
@@ -365,29 +378,39 @@ static int setup_tb(mmsp_gpu_handle* h)
     char* p = static_cast<char*>(h->work);
     h->tb_inst = reinterpret_cast<pf::BatchInst*>(p);
     p += align256(sizeof(pf::BatchInst));
-    h->tb_list = reinterpret_cast<pf::TbItem*>(p);
-    p += align256(sizeof(pf::TbItem) * items.size());
-    h->tb_counters = reinterpret_cast<int*>(p);
-    h->tb_items = (int)items.size();
-    const bool aligned = n1 % 4 == 0;   // 16-byte row groups
-    h->tb_fn = aligned ? pf::tb_kernel(0, pf::kTbAnyDepth, h->d.model, h->c.unit_w)
-                       : pf::tb_kernel_any(h->d.model, h->c.unit_w);
-    h->tb_smem = pf::tb_smem(0);
-    // Queued on the handle's stream, ahead of its first launch, with no
-    // synchronisation: a server request's stream may carry another request's
-    // queued steps.  A copy from pageable memory has staged its source when
-    // the call returns, so the host arrays may go out of scope.
     cudaError_t e = cudaMemcpyAsync(h->tb_inst, &bi, sizeof(bi), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h->tb_list, items.data(), sizeof(pf::TbItem) * items.size(), cudaMemcpyHostToDevice,
-                            h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->tb_counters, 0, 256, h->stream);
-    if (e == cudaSuccess) e = pf::ensure_smem(h->tb_fn, h->tb_smem);
-    int per_sm = 0;
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, h->tb_fn, pf::kTbShapes[0].nt, h->tb_smem);
+    h->tb_strips = tb_strips(&h->d);
+    if (h->tb_strips) {
+        std::vector<pf::StripItem> items;
+        pf::strip_items(0, n0, n1, pf::strip_rows(n0, n1), &items);
+        h->tb_strip_list = reinterpret_cast<pf::StripItem*>(p);
+        h->tb_items = (int)items.size();
+        h->tb_fn = pf::strip_kernel(h->d.model, h->c.unit_w, aligned);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p, items.data(), sizeof(pf::StripItem) * items.size(), cudaMemcpyHostToDevice,
+                                h->stream);
+    } else {
+        const int TX = tb_tile_rows(), TZ = tb_tile_cols();
+        std::vector<pf::TbItem> items;
+        for (int x0 = 0; x0 < n0; x0 += TX)
+            for (int z0 = 0; z0 < n1; z0 += TZ)
+                items.push_back(pf::TbItem{0, x0, z0, std::min(TX, n0 - x0), std::min(TZ, n1 - z0)});
+        h->tb_list = reinterpret_cast<pf::TbItem*>(p);
+        h->tb_items = (int)items.size();
+        h->tb_counters = reinterpret_cast<int*>(p + align256(sizeof(pf::TbItem) * items.size()));
+        h->tb_fn = aligned ? pf::tb_kernel(0, pf::kTbAnyDepth, h->d.model, h->c.unit_w)
+                           : pf::tb_kernel_any(h->d.model, h->c.unit_w);
+        h->tb_smem = pf::tb_smem(0);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p, items.data(), sizeof(pf::TbItem) * items.size(), cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->tb_counters, 0, 256, h->stream);
+        if (e == cudaSuccess) e = pf::ensure_smem(h->tb_fn, h->tb_smem);
+        int per_sm = 0;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, h->tb_fn, pf::kTbShapes[0].nt, h->tb_smem);
+        h->tb_blocks = std::max(1, std::min(per_sm * pf::sm_count(), h->tb_items));
+    }
     if (e != cudaSuccess) return cuda_fail(h, e, "blocked kernel setup");
-    h->tb_blocks = std::max(1, std::min(per_sm * pf::sm_count(), h->tb_items));
     h->tb_launches = 0;
     h->tb = true;
     return MMSP_GPU_OK;
@@ -396,9 +419,12 @@ static int setup_tb(mmsp_gpu_handle* h)
 // kTbAnyDepth steps from buf[cur] in one launch of the blocked kernel.
 static cudaError_t tb_launch(mmsp_gpu_handle* h, cudaStream_t s)
 {
+    const void* in = h->buf[h->cur];
+    void* out = h->buf[h->cur ^ 1];
     const cudaError_t e =
-        pf::launch_tb(h->tb_fn, h->tb_blocks, pf::kTbShapes[0].nt, h->tb_smem, h->tb_inst, h->tb_list, h->tb_items,
-                      h->buf[h->cur], h->buf[h->cur ^ 1], h->tb_counters, (int)(h->tb_launches & 1), s);
+        h->tb_strips ? pf::launch_strips(h->tb_fn, h->tb_inst, h->tb_strip_list, h->tb_items, in, out, s)
+                     : pf::launch_tb(h->tb_fn, h->tb_blocks, pf::kTbShapes[0].nt, h->tb_smem, h->tb_inst, h->tb_list,
+                                     h->tb_items, in, out, h->tb_counters, (int)(h->tb_launches & 1), s);
     h->cur ^= 1;
     h->tb_launches++;
     return e;

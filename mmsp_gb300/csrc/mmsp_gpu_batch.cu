@@ -42,8 +42,25 @@ struct Member {
 
 struct Tuning {
     int rows = 0, threads = 0;   // per-step kernel: rows per work item, block size
-    int ks = 0, shape = 0;       // temporally blocked kernel: steps per launch (0: not used), region shape
+    int ks = 0, shape = 0;       // temporally blocked kernels: steps per launch (0: not used), region shape
 };
+
+// Region shapes of the tile kernel come first; those from kTbShapeCount on are
+// the strip kernel's, by rows per strip.  256 grids of sides 64-512, us per
+// step: strips of 16 rows 29.5, 32 rows 22.9, 56 rows 21.0, 72 rows 19.4, 104
+// rows 19.9, 136 rows 20.6, against 25.1 for the best tile (96 x 128); batches
+// of few or small grids want the short ones.
+const int kStripRows[] = {4, 8, 16, 24, 32, 40, 56, 72, 104, 136};
+const int kShapes = kTbShapeCount + (int)(sizeof(kStripRows) / sizeof(kStripRows[0]));
+bool shape_strips(int shape) { return shape >= kTbShapeCount; }
+// Is (steps per launch, shape) a kernel that is built?
+bool shape_ok(int ks, int shape)
+{
+    if (shape < 0 || shape >= kShapes) return false;
+    if (shape_strips(shape)) return ks == kStripKS;
+    return std::find(std::begin(kTbDepths), std::end(kTbDepths), ks) != std::end(kTbDepths) &&
+           4 * ks < std::min(kTbShapes[shape].ri, kTbCols);   // leaves an interior
+}
 
 std::mutex g_tune_mu;
 std::map<std::string, Tuning> g_tune;   // batch shape -> tuning
@@ -71,7 +88,8 @@ struct mmsp_gpu_batch {
     Tuning tune;
     // temporally blocked kernel (FP32 batches of persistent grids only)
     TbItem* d_tb;
-    int tb_nitems, tb_cap, tb_blocks;
+    StripItem* d_strips;
+    int tb_nitems, tb_cap, strips_cap, tb_blocks;
     bool tuned, tuned_from_cache;
     double tune_ms;
     int blocks;
@@ -103,6 +121,7 @@ static void brelease(mmsp_gpu_batch* b)
     if (b->d_insts) cudaFree(b->d_insts);
     if (b->d_items) cudaFree(b->d_items);
     if (b->d_tb) cudaFree(b->d_tb);
+    if (b->d_strips) cudaFree(b->d_strips);
     if (b->own) cudaStreamDestroy(b->own);
 }
 
@@ -368,7 +387,7 @@ static int set_items(mmsp_gpu_batch* b, int rows, int threads)
     return MMSP_GPU_OK;
 }
 
-// The temporally blocked kernel applies when every grid of an FP32 batch
+// The temporally blocked kernels apply when every grid of an FP32 batch
 // joins the persistent kernel (grids with their own plans advance one step
 // per launch).
 static bool tb_possible(const mmsp_gpu_batch* b)
@@ -376,44 +395,65 @@ static bool tb_possible(const mmsp_gpu_batch* b)
     return b->dtype == MMSP_GPU_F32 && b->npersistent > 0 && b->npersistent == (int)b->m.size();
 }
 
-// Tiles of every grid for region shape `shape` and depth `ks`, largest first.
-static int set_tb(mmsp_gpu_batch* b, int shape, int ks)
+// A list of items on the device, its buffer grown where needed.
+template <typename Item>
+static int set_list(mmsp_gpu_batch* b, const std::vector<Item>& items, Item** list, int* cap)
 {
-    const int H = 2 * ks;
-    const int TX = kTbShapes[shape].ri - 2 * H, TZ = kTbCols - 2 * H;
-    for (const auto& bi : b->insts)   // 16-byte groups: rows of a multiple of 4 cells at 16-byte aligned offsets
-        if (bi.n1 % 4 || bi.off % 4) return bfail(b, MMSP_GPU_EUNSUPPORTED, "tile kernel alignment");
-    std::vector<TbItem> items;
-    for (int i = 0; i < (int)b->insts.size(); i++) {
-        const int n0 = b->insts[i].n0, n1 = b->insts[i].n1;
-        for (int x0 = 0; x0 < n0; x0 += TX)
-            for (int z0 = 0; z0 < n1; z0 += TZ)
-                items.push_back(TbItem{i, x0, z0, std::min(TX, n0 - x0), std::min(TZ, n1 - z0)});
-    }
-    std::stable_sort(items.begin(), items.end(),
-                     [](const TbItem& a, const TbItem& c) { return a.tx * a.tz > c.tx * c.tz; });
-    if ((int)items.size() > b->tb_cap) {
-        if (b->d_tb) cudaFree(b->d_tb);
-        b->d_tb = nullptr;
-        b->tb_cap = 0;
-        if (cudaMalloc((void**)&b->d_tb, sizeof(TbItem) * items.size()) != cudaSuccess) {
+    if ((int)items.size() > *cap) {
+        if (*list) cudaFree(*list);
+        *list = nullptr;
+        *cap = 0;
+        if (cudaMalloc((void**)list, sizeof(Item) * items.size()) != cudaSuccess) {
             cudaGetLastError();
             return bfail(b, MMSP_GPU_ENOMEM, "tile list");
         }
-        b->tb_cap = (int)items.size();
+        *cap = (int)items.size();
     }
-    cudaError_t e = cudaMemcpyAsync(b->d_tb, items.data(), sizeof(TbItem) * items.size(), cudaMemcpyHostToDevice,
+    cudaError_t e = cudaMemcpyAsync(*list, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice,
                                     b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return bcuda(b, e, "tile list upload");
-    const void* fn = tb_kernel(shape, ks, b->persistent_model, b->unit);
-    const size_t smem = tb_smem(shape);
-    if ((e = ensure_smem(fn, smem)) != cudaSuccess) return bcuda(b, e, "tile kernel shared memory");
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTbShapes[shape].nt, smem)) != cudaSuccess)
-        return bcuda(b, e, "occupancy");
-    b->tb_blocks = std::max(1, per_sm) * sm_count();
     b->tb_nitems = (int)items.size();
+    return MMSP_GPU_OK;
+}
+
+// Tiles of every grid for region shape `shape` and depth `ks`, largest first,
+// or the windows of their strips.
+static int set_tb(mmsp_gpu_batch* b, int shape, int ks)
+{
+    for (const auto& bi : b->insts)   // 16-byte groups: rows of a multiple of 4 cells at 16-byte aligned offsets
+        if (bi.n1 % 4 || bi.off % 4) return bfail(b, MMSP_GPU_EUNSUPPORTED, "tile kernel alignment");
+    int rc;
+    if (shape_strips(shape)) {
+        std::vector<StripItem> items;
+        for (int i = 0; i < (int)b->insts.size(); i++)
+            strip_items(i, b->insts[i].n0, b->insts[i].n1, kStripRows[shape - kTbShapeCount], &items);
+        // longest first, so the tail is short items
+        std::stable_sort(items.begin(), items.end(),
+                         [](const StripItem& a, const StripItem& c) { return a.rows > c.rows; });
+        if ((rc = set_list(b, items, &b->d_strips, &b->strips_cap))) return rc;
+    } else {
+        const int H = 2 * ks;
+        const int TX = kTbShapes[shape].ri - 2 * H, TZ = kTbCols - 2 * H;
+        std::vector<TbItem> items;
+        for (int i = 0; i < (int)b->insts.size(); i++) {
+            const int n0 = b->insts[i].n0, n1 = b->insts[i].n1;
+            for (int x0 = 0; x0 < n0; x0 += TX)
+                for (int z0 = 0; z0 < n1; z0 += TZ)
+                    items.push_back(TbItem{i, x0, z0, std::min(TX, n0 - x0), std::min(TZ, n1 - z0)});
+        }
+        std::stable_sort(items.begin(), items.end(),
+                         [](const TbItem& a, const TbItem& c) { return a.tx * a.tz > c.tx * c.tz; });
+        if ((rc = set_list(b, items, &b->d_tb, &b->tb_cap))) return rc;
+        const void* fn = tb_kernel(shape, ks, b->persistent_model, b->unit);
+        const size_t smem = tb_smem(shape);
+        cudaError_t e;
+        if ((e = ensure_smem(fn, smem)) != cudaSuccess) return bcuda(b, e, "tile kernel shared memory");
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTbShapes[shape].nt, smem)) != cudaSuccess)
+            return bcuda(b, e, "occupancy");
+        b->tb_blocks = std::max(1, per_sm) * sm_count();
+    }
     b->tune.ks = ks;
     b->tune.shape = shape;
     if (b->graph) {
@@ -427,11 +467,13 @@ static int set_tb(mmsp_gpu_batch* b, int shape, int ks)
 static cudaError_t step_tb(mmsp_gpu_batch* b, cudaStream_t s, int in, int out)
 {
     const int parity = (int)(b->launches & 1);
-    cudaError_t e = launch_tb(tb_kernel(b->tune.shape, b->tune.ks, b->persistent_model, b->unit), b->tb_blocks,
-                              kTbShapes[b->tune.shape].nt, tb_smem(b->tune.shape), b->d_insts, b->d_tb, b->tb_nitems,
-                              b->pool[in], b->pool[out], b->counters, parity, s);
     b->launches++;
-    return e;
+    if (shape_strips(b->tune.shape))
+        return launch_strips(strip_kernel(b->persistent_model, b->unit, true), b->d_insts, b->d_strips, b->tb_nitems,
+                             b->pool[in], b->pool[out], s);
+    return launch_tb(tb_kernel(b->tune.shape, b->tune.ks, b->persistent_model, b->unit), b->tb_blocks,
+                     kTbShapes[b->tune.shape].nt, tb_smem(b->tune.shape), b->d_insts, b->d_tb, b->tb_nitems,
+                     b->pool[in], b->pool[out], b->counters, parity, s);
 }
 
 // One step from pool `in` to pool `out`.
@@ -493,7 +535,7 @@ static void load_cache_file()
     char line[512];
     while (fgets(line, sizeof line, f))
         if (sscanf(line, " \"%127[^\"]\" : [ %d , %d , %d , %d ]", key, &t.rows, &t.threads, &t.ks, &t.shape) == 5 &&
-            t.rows > 0 && t.threads > 0 && t.ks >= 0 && t.shape >= 0 && t.shape < kTbShapeCount)
+            t.rows > 0 && t.threads > 0 && (t.ks == 0 || shape_ok(t.ks, t.shape)))
             g_tune[key] = t;
     fclose(f);
 }
@@ -543,8 +585,7 @@ extern "C" int mmsp_gpu_batch_tune(mmsp_gpu_batch* b, int force)
         t.rows = 16;
         t.threads = 128;
         if (sscanf(fix, "%d,%d", &t.ks, &t.shape) == 2 && t.shape >= 0 && t.shape < kTbShapeCount &&
-            (t.ks == 0 || std::find(std::begin(kTbDepths), std::end(kTbDepths), t.ks) != std::end(kTbDepths)) &&
-            4 * t.ks < std::min(kTbShapes[t.shape].ri, kTbCols)) {
+            (t.ks == 0 || shape_ok(t.ks, t.shape))) {
             int rc = apply_tuning(b, t);
             if (rc) return rc;
             b->tuned = true;
@@ -567,7 +608,7 @@ extern "C" int mmsp_gpu_batch_tune(mmsp_gpu_batch* b, int force)
         }
     }
     // Candidates: the per-step kernel's rows per work item x threads per
-    // block, then (FP32 batches) the temporally blocked kernel's region shape
+    // block, then (FP32 batches) the temporally blocked kernels' region shape
     // x steps per launch.  Each is timed on the live state (pool cur -> idle
     // pool, so the state is not changed) and scored per step.
     static const int kRows[] = {4, 8, 16, 32, 64};
@@ -610,9 +651,9 @@ extern "C" int mmsp_gpu_batch_tune(mmsp_gpu_batch* b, int force)
             }
         }
     if (tb_possible(b)) {
-        for (int shape = 0; shape < kTbShapeCount; shape++)
+        for (int shape = 0; shape < kShapes; shape++)
             for (int ks : kTbDepths) {
-                if (2 * 2 * ks >= std::min(kTbShapes[shape].ri, kTbCols)) continue;   // no interior
+                if (!shape_ok(ks, shape)) continue;
                 if ((rc = set_tb(b, shape, ks))) goto done;
                 float ms = 0;
                 e = time2([&] { return step_tb(b, b->stream, b->cur, b->cur ^ 1); }, &ms);
@@ -763,12 +804,14 @@ extern "C" int mmsp_gpu_batch_get_info(const mmsp_gpu_batch* b, mmsp_gpu_batch_i
     info->tuned_from_cache = b->tuned_from_cache ? 1 : 0;
     info->tune_ms = b->tune_ms;
     info->temporal_depth = b->tune.ks > 0 ? b->tune.ks : 1;
-    info->tile_rows = b->tune.ks > 0 ? kTbShapes[b->tune.shape].ri : 0;
+    info->tile_rows = b->tune.ks == 0               ? 0
+                      : shape_strips(b->tune.shape) ? kStripRows[b->tune.shape - kTbShapeCount] + 4 * kStripKS
+                                                    : kTbShapes[b->tune.shape].ri;
     info->tile_cols = b->tune.ks > 0 ? kTbCols : 0;
     info->tiles = b->tune.ks > 0 ? b->tb_nitems : 0;
     info->device_bytes = 2 * (size_t)b->pool_elems * b->esize + kPartialsBytes + 256 +
                          sizeof(BatchInst) * b->insts.size() + sizeof(BatchItem) * b->items_cap +
-                         sizeof(TbItem) * b->tb_cap;
+                         sizeof(TbItem) * b->tb_cap + sizeof(StripItem) * b->strips_cap;
     return MMSP_GPU_OK;
 }
 

@@ -112,6 +112,15 @@ static __device__ __forceinline__ void cp_async16(void* dst, const void* src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
+// Close a group of this thread's cp.async copies; wait until all but its last
+// N groups have landed.
+static __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+static __device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Wait until this thread's earlier cp.async copies have landed.
 static __device__ __forceinline__ void cp_async_wait_all()
 {

@@ -15,6 +15,8 @@
 //
 // FP64 instances use the reference's operation order (bit-identical to the
 // single-grid kernels and the oracle); FP32 instances use ordinary operators.
+#include <algorithm>
+
 #include "pf_async.cuh"
 #include "pf_batch.h"
 #include "pf_device.cuh"
@@ -484,6 +486,204 @@ cudaError_t launch_tb(const void* fn, int blocks, int threads, size_t smem, cons
     void* args[] = {(void*)&insts, (void*)&items, (void*)&nitems, (void*)&in, (void*)&out, (void*)&counters,
                     (void*)&parity};
     return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, smem, s);
+}
+
+// ---------------------------------------------------------------------------
+// Temporal blocking in registers: kStripKS steps per launch, one independent
+// warp per window of a strip of rows.
+//
+// A warp streams the rows of its strip through kStripKS stages, one per step.
+// A stage holds c of two rows and mu of two rows (4 cells per lane); given the
+// next row of its step it computes mu one row up, advances the row two up and
+// leaves it for the next stage.  Nothing goes through shared memory between
+// lanes and no barrier is met: a strip of L rows reads L + 16 rows (two a side
+// per step) and writes L, and a row costs its arithmetic, one load and one
+// store for four steps.  Left and right neighbours come from the adjacent lanes;
+// the outer 8 columns of a window's 128 are the halo of the four steps.
+//
+// Rows of any length: a strip's rows are virtual rows of n1 + 16 cells (the
+// halo included, wrapped periodically on load; rounded up to a multiple of 4),
+// and the windows run over the virtual rows of all strips of a grid without a
+// gap, 112 cells each.  Where rows are a multiple of 4 cells a lane's group is
+// one 16-byte load and store, else four single cells.  The last strip starts
+// at n0 - L and writes some rows twice, with the same values.  Per cell the
+// operations are those of the tile kernel above, so the two agree bit for bit.
+//
+// What bounds it: a round (one row through the four stages) takes a quarter of
+// an SM 316-330 cycles however many warps share it; instructions issue in 60%
+// of cycles and the wide FP32 pipe is 63% busy at 4096 x 4096.  Against the
+// tile kernel, whose steps meet a barrier and pass every cell through shared
+// memory, us per step, before -> after: 4096^2 15.3 -> 11.6, 1024^2 2.46 ->
+// 1.97, 553^2 2.23 -> 1.75, 256^2 1.98 -> 1.43, 64^2 1.87 -> 1.33.  Four rows
+// an iteration: 11.3 us at 4096^2 against 14.8 with one, 12.6 with two and 11.2
+// with nine, whose remainder costs short strips more.  Three blocks an SM: 155
+// registers; a fourth block spills.
+template <int MODEL, bool UNIT>
+struct StripStage {
+    float4 cA, cB, mA, mB;   // c of rows j-2, j-1; mu of rows j-3, j-2
+    __device__ __forceinline__ float4 next(float4 c, float w0, float w1, float kappa, float neg_r, float u, float dtm)
+    {
+        const float4 m = tb_mu4<MODEL, UNIT>(cA, cB, c, w0, w1, kappa, neg_r, u);
+        const float4 o = tb_update4<UNIT>(cA, mA, mB, m, w0, w1, dtm);
+        cA = cB;
+        cB = c;
+        mA = mB;
+        mB = m;
+        return o;
+    }
+};
+
+template <int MODEL, bool UNIT, bool ALIGNED>
+__global__ void __launch_bounds__(kStripThreads, 3)
+ch2_strip_kernel(const BatchInst* __restrict__ insts, const StripItem* __restrict__ items, int nitems,
+                 const float* __restrict__ in, float* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    const int w = (int)((blockIdx.x * kStripThreads + threadIdx.x) >> 5);
+    if (w >= nitems) return;   // whole warps
+    const StripItem it = items[w];
+    const BatchInst bi = insts[it.inst];
+    const int n0 = bi.n0, n1 = bi.n1, L = it.rows;
+    const float kappa = (float)bi.kappa, dtm = (float)bi.dtm, neg_r = (float)bi.neg_r, u = (float)bi.u;
+    const float w0 = (float)bi.w0, w1 = (float)bi.w1;
+    const int vg = (n1 + 16 + 3) >> 2, total = it.strips * vg;   // groups of 4 cells
+    const int gi = it.window * kStripUse + lane - 2;
+    const int gc = min(max(gi, 0), total - 1);
+    const int strip = gc / vg, zz = 4 * (gc - strip * vg) - 8;
+    const bool mine = lane >= 2 && lane < 30 && gi < total;
+    const int row0 = min(strip * L, n0 - L);
+    int z[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) z[q] = wrapi(zz + q, n1);   // (ALIGNED: z[0] .. z[0]+3)
+    const float* base = in + bi.off;
+    const long long wrap = (long long)n0 * n1;
+    int r = wrapi(row0 - 8, n0);
+    const float* p = base + (long long)r * n1;
+    // rows on their way, kStripRing - 1 ahead: each lane copies and reads its own
+    // cells, so its own copies are all it waits for
+    __shared__ float4 s_ring[kStripThreads / 32][kStripRing][32];
+    float4(*ring)[32] = s_ring[threadIdx.x >> 5];
+    int slot_in = 0, slot_out = 0;
+    auto fetch = [&]() {
+        float* d = reinterpret_cast<float*>(&ring[slot_in][lane]);
+        if (ALIGNED) {
+            cp_async16(d, p + z[0]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) cp_async4(d + q, p + z[q]);
+        }
+        cp_async_commit();
+        slot_in = (slot_in + 1) & (kStripRing - 1);
+        p += n1;
+        if (++r == n0) {
+            r = 0;
+            p -= wrap;
+        }
+    };
+    auto pull = [&]() {
+        cp_async_wait<kStripRing - 2>();
+        const float4 v = ring[slot_out][lane];
+        slot_out = (slot_out + 1) & (kStripRing - 1);
+        fetch();
+        return v;
+    };
+#pragma unroll
+    for (int i = 0; i < kStripRing - 1; i++) fetch();
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    StripStage<MODEL, UNIT> s1{zero, zero, zero, zero}, s2 = s1, s3 = s1, s4 = s1;
+    // Each stage takes what the stage before made in the previous round, so the
+    // four are independent of each other within a round.
+    float4 o1 = zero, o2 = zero, o3 = zero;
+#define PF_STAGE(s, v) s.next(v, w0, w1, kappa, neg_r, u, dtm)
+    // a stage starts with the first valid row of the one before: 4 rounds and one in flight
+#pragma unroll 1
+    for (int i = 0; i < kStripLead; i++) {
+        const float4 v = pull();
+        if (i >= 15) PF_STAGE(s4, o3);
+        if (i >= 10) o3 = PF_STAGE(s3, o2);
+        if (i >= 5) o2 = PF_STAGE(s2, o1);
+        o1 = PF_STAGE(s1, v);
+    }
+    float* dst = out + bi.off + (long long)row0 * n1 + zz;
+    const bool ok = mine && zz >= 0 && zz < n1;
+#pragma unroll 4
+    for (int i = 0; i < L; i++) {
+        const float4 v = pull();
+        const float4 o4 = PF_STAGE(s4, o3);
+        o3 = PF_STAGE(s3, o2);
+        o2 = PF_STAGE(s2, o1);
+        o1 = PF_STAGE(s1, v);
+        if (ALIGNED) {
+            if (ok) *reinterpret_cast<float4*>(dst) = o4;
+        } else if (mine && zz > -4) {
+            if (zz >= 0 && zz < n1) dst[0] = o4.x;
+            if (zz + 1 >= 0 && zz + 1 < n1) dst[1] = o4.y;
+            if (zz + 2 >= 0 && zz + 2 < n1) dst[2] = o4.z;
+            if (zz + 3 >= 0 && zz + 3 < n1) dst[3] = o4.w;
+        }
+        dst += n1;
+    }
+    cp_async_wait<0>();
+#undef PF_STAGE
+}
+
+template <int MODEL, bool UNIT>
+static const void* strip_pick(bool aligned)
+{
+    return aligned ? (const void*)&ch2_strip_kernel<MODEL, UNIT, true>
+                   : (const void*)&ch2_strip_kernel<MODEL, UNIT, false>;
+}
+
+const void* strip_kernel(int model, bool unit, bool aligned)
+{
+    if (model == MMSP_GPU_CH)
+        return unit ? strip_pick<MMSP_GPU_CH, true>(aligned) : strip_pick<MMSP_GPU_CH, false>(aligned);
+    return unit ? strip_pick<MMSP_GPU_CH_POLY, true>(aligned) : strip_pick<MMSP_GPU_CH_POLY, false>(aligned);
+}
+
+// Strips of `rows` rows made as even as n0 allows (the rows of the last one
+// that the one before has written already are work done twice).
+static int even_rows(int n0, int rows)
+{
+    const int want = std::max(1, (n0 + rows / 2) / rows);
+    return (n0 + want - 1) / want;
+}
+
+long long strip_windows(int n0, int n1, int rows)
+{
+    const int L = even_rows(n0, rows);
+    const long long groups = (long long)((n0 + L - 1) / L) * ((n1 + 16 + 3) / 4);
+    return (groups + kStripUse - 1) / kStripUse;
+}
+
+void strip_items(int inst, int n0, int n1, int rows, std::vector<StripItem>* items)
+{
+    const int L = even_rows(n0, rows), strips = (n0 + L - 1) / L;
+    const int windows = (int)strip_windows(n0, n1, rows);
+    for (int w = 0; w < windows; w++) items->push_back(StripItem{inst, w, L, strips});
+}
+
+int strip_rows(int n0, int n1)
+{
+    constexpr long long wave = 152 * (kStripThreads / 32);   // quarters of the chip's SMs; the footprint needs no device
+    int best = 1;
+    long long cost = 0;
+    for (int rows = 1; rows <= std::min(n0, 256); rows++) {
+        const long long c = (strip_windows(n0, n1, rows) + wave - 1) / wave * (even_rows(n0, rows) + kStripLead);
+        if (cost == 0 || c < cost) {
+            cost = c;
+            best = rows;
+        }
+    }
+    return best;
+}
+
+cudaError_t launch_strips(const void* fn, const BatchInst* insts, const StripItem* items, int nitems, const void* in,
+                          void* out, cudaStream_t s)
+{
+    constexpr int per = kStripThreads / 32;
+    void* args[] = {(void*)&insts, (void*)&items, (void*)&nitems, (void*)&in, (void*)&out};
+    return cudaLaunchKernel(fn, dim3((nitems + per - 1) / per), dim3(kStripThreads), args, 0, s);
 }
 
 }  // namespace pf

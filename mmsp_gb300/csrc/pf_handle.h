@@ -9,6 +9,7 @@
 namespace pf {
 struct BatchInst;
 struct TbItem;
+struct StripItem;
 // Device bytes of one block holding a handle's buffers (two states, the
 // reduction partials, the error words, a model's work grid), each 256-byte
 // aligned, for create_in.
@@ -52,14 +53,16 @@ struct mmsp_gpu_handle {
     pf::Ch64Steps ch64s;
     unsigned multi_base;
     // 2D FP32 Cahn-Hilliard: blocks of pf::kTbAnyDepth steps per launch of the
-    // temporally blocked kernel (its instance, tile list and work counters in `work`)
-    bool tb;
+    // strip kernel, or for few rows the tile kernel (the instance, the list of
+    // strip windows or tiles and the tile kernel's work counters in `work`)
+    bool tb, tb_strips;
     const void* tb_fn;
     size_t tb_smem;
     int tb_blocks, tb_items;
     int64_t tb_launches;     // launches so far: their parity picks the work counter
     pf::BatchInst* tb_inst;
     pf::TbItem* tb_list;
+    pf::StripItem* tb_strip_list;
     int* tb_counters;
     char err[512];
 };
