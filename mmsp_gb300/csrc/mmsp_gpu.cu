@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -35,6 +36,7 @@ static int cuda_fail(mmsp_gpu_handle* h, cudaError_t e, const char* where)
 }
 
 static int check_flags(mmsp_gpu_handle* h);
+static int report_flags(mmsp_gpu_handle* h, const int* f);
 
 extern "C" int mmsp_gpu_version(void) { return MMSP_GPU_ABI_VERSION; }
 
@@ -258,19 +260,133 @@ extern "C" int mmsp_gpu_footprint(const mmsp_gpu_desc* d, size_t* bytes)
     return MMSP_GPU_OK;
 }
 
-static void release(mmsp_gpu_handle* h)
+// What a handle of its own takes from the device: one block for states and
+// scratch, a stream, the two events of its step clock.  mmsp_gpu_destroy gives
+// a set back once the handle's work is done, and the next create takes it:
+// update() of a little grid spent most of its time in five cudaMallocs and
+// their cudaFrees, which map and unmap memory.  update() of 64 x 64 FP64 cells
+// by 20 steps, host to host: 306 us before, 121 with the sets.
+// At most kKits sets of at most kKitBytes each are held (64 MB), the one given
+// back longest ago going first, and all of them are freed when an allocation
+// fails; larger blocks are freed with their handle.  A set goes to handles of
+// the CUDA context that made it only: its identifier is never used again, so a
+// set that a device reset took away is dropped unread.
+struct Kit {
+    unsigned long long ctx;   // 0: not known
+    size_t bytes;
+    void* block;
+    cudaStream_t stream;
+    cudaEvent_t ev0, ev1;
+};
+static const size_t kKits = 8, kKitBytes = 8u << 20;
+static std::mutex g_kits_mu;
+static std::vector<Kit> g_kits;
+
+static unsigned long long context_id()
+{
+    typedef int (*CtxGetId)(void*, unsigned long long*);
+    static const CtxGetId get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (CtxGetId)f;
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == 0 ? id : 0;   // null: the calling thread's context
+}
+
+static void free_kit(const Kit& k)
+{
+    if (k.ev0) cudaEventDestroy(k.ev0);
+    if (k.ev1) cudaEventDestroy(k.ev1);
+    if (k.block) cudaFree(k.block);
+    if (k.stream) cudaStreamDestroy(k.stream);
+}
+
+// The held sets of context `ctx` (0: none), out of the list.
+static std::vector<Kit> drain_kits(unsigned long long ctx)
+{
+    std::vector<Kit> mine;
+    std::lock_guard<std::mutex> lock(g_kits_mu);
+    for (size_t i = 0; ctx && i < g_kits.size();) {
+        if (g_kits[i].ctx != ctx) {
+            i++;
+            continue;
+        }
+        mine.push_back(g_kits[i]);
+        g_kits.erase(g_kits.begin() + i);
+    }
+    return mine;
+}
+
+static cudaError_t take_kit(size_t bytes, Kit* kit)
+{
+    const unsigned long long ctx = context_id();
+    if (ctx && bytes <= kKitBytes) {
+        std::lock_guard<std::mutex> lock(g_kits_mu);
+        size_t best = g_kits.size();
+        for (size_t i = 0; i < g_kits.size(); i++)
+            if (g_kits[i].ctx == ctx && g_kits[i].bytes >= bytes &&
+                (best == g_kits.size() || g_kits[i].bytes < g_kits[best].bytes))
+                best = i;
+        if (best < g_kits.size()) {
+            *kit = g_kits[best];
+            g_kits.erase(g_kits.begin() + best);
+            return cudaSuccess;
+        }
+    }
+    *kit = Kit{0, bytes, nullptr, nullptr, nullptr, nullptr};
+    cudaError_t e = cudaStreamCreateWithFlags(&kit->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreate(&kit->ev0);
+    if (e == cudaSuccess) e = cudaEventCreate(&kit->ev1);
+    if (e == cudaSuccess) e = cudaMalloc(&kit->block, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        const std::vector<Kit> held = drain_kits(context_id());
+        for (const Kit& k : held) free_kit(k);
+        if (!held.empty() && kit->ev1) {
+            cudaGetLastError();
+            e = cudaMalloc(&kit->block, bytes);
+        }
+    }
+    if (e == cudaSuccess) {
+        kit->ctx = context_id();
+        return e;
+    }
+    cudaGetLastError();
+    free_kit(*kit);
+    return e;
+}
+
+// `idle`: nothing that uses the set is queued or running.
+static void give_kit(Kit kit, bool idle)
+{
+    if (idle && kit.ctx && kit.ctx == context_id() && kit.bytes <= kKitBytes) {
+        std::lock_guard<std::mutex> lock(g_kits_mu);
+        g_kits.push_back(kit);
+        if (g_kits.size() <= kKits) return;
+        size_t i = 0;
+        while (g_kits[i].ctx != kit.ctx) i++;   // another context's is not this thread's to free
+        kit = g_kits[i];
+        g_kits.erase(g_kits.begin() + i);
+    }
+    free_kit(kit);
+}
+
+// `idle` as for give_kit.
+static void release(mmsp_gpu_handle* h, bool idle = false)
 {
     if (h->out) pf::output_release(h);   // waits for snapshots still being written
     if (h->graph) cudaGraphExecDestroy(h->graph);
-    if (h->ev0) cudaEventDestroy(h->ev0);
-    if (h->ev1) cudaEventDestroy(h->ev1);
-    if (h->external) return;   // the caller's block and stream
-    if (h->buf[0]) cudaFree(h->buf[0]);
-    if (h->buf[1]) cudaFree(h->buf[1]);
-    if (h->partials) cudaFree(h->partials);
-    if (h->work) cudaFree(h->work);
-    if (h->flags) cudaFree(h->flags);
-    if (h->own) cudaStreamDestroy(h->own);
+    if (h->external) {   // the caller's block and stream
+        if (h->ev0) cudaEventDestroy(h->ev0);
+        if (h->ev1) cudaEventDestroy(h->ev1);
+        return;
+    }
+    give_kit(Kit{h->kit_ctx, h->kit_bytes, h->buf[0], h->own, h->ev0, h->ev1}, idle);
 }
 
 size_t pf::handle_block_bytes(const mmsp_gpu_desc& d)
@@ -281,16 +397,11 @@ size_t pf::handle_block_bytes(const mmsp_gpu_desc& d)
 static int make_plan(mmsp_gpu_handle* h);
 static int setup_tb(mmsp_gpu_handle* h);
 
-int pf::create_in(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc, void* block, cudaStream_t stream)
+static mmsp_gpu_handle* new_handle(const mmsp_gpu_desc* desc)
 {
-    if (!out || !block || ((uintptr_t)block & 255)) return MMSP_GPU_EINVAL;
-    *out = nullptr;
-    int rc = validate(desc, nullptr, 0);
-    if (rc) return rc;
     mmsp_gpu_handle* h = new (std::nothrow) mmsp_gpu_handle();
-    if (!h) return MMSP_GPU_ENOMEM;
+    if (!h) return nullptr;
     memset(h, 0, sizeof(*h));
-    h->external = true;
     h->d = *desc;
     for (int a = desc->dim; a < 3; a++) h->d.n[a] = 1;
     h->g = pf::make_geom(h->d);
@@ -299,7 +410,14 @@ int pf::create_in(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc, void* block,
     h->esize = esize_of(&h->d);
     h->bytes = state_bytes(&h->d);
     h->elems = h->bytes / h->esize;
-    h->own = h->stream = stream;
+    return h;
+}
+
+// Lay the handle out in `block` (handle_block_bytes) and plan its steps, on its
+// stream.  The status words lie behind the reduction's results, so one copy
+// reads both.
+static int set_up(mmsp_gpu_handle* h, void* block)
+{
     char* p = static_cast<char*>(block);
     h->buf[0] = p;
     p += align256(h->bytes);
@@ -310,17 +428,29 @@ int pf::create_in(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc, void* block,
     h->flags = reinterpret_cast<int*>(p);
     p += 256;
     if (work_bytes(&h->d)) h->work = p;
-    cudaError_t e = cudaEventCreate(&h->ev0);
-    if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->flags, 0, 256, stream);
-    if (e != cudaSuccess) {
+    if (cudaMemsetAsync(h->flags, 0, 256, h->stream) != cudaSuccess) {
         cudaGetLastError();
-        release(h);
-        delete h;
         return MMSP_GPU_ECUDA;
     }
-    rc = make_plan(h);
-    if (!rc) rc = setup_tb(h);
+    const int rc = make_plan(h);
+    return rc ? rc : setup_tb(h);
+}
+
+int pf::create_in(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc, void* block, cudaStream_t stream)
+{
+    if (!out || !block || ((uintptr_t)block & 255)) return MMSP_GPU_EINVAL;
+    *out = nullptr;
+    int rc = validate(desc, nullptr, 0);
+    if (rc) return rc;
+    mmsp_gpu_handle* h = new_handle(desc);
+    if (!h) return MMSP_GPU_ENOMEM;
+    h->external = true;
+    h->own = h->stream = stream;
+    if (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess) {
+        cudaGetLastError();
+        rc = MMSP_GPU_ECUDA;
+    }
+    if (!rc) rc = set_up(h, block);
     if (rc) {
         release(h);
         delete h;
@@ -441,33 +571,20 @@ extern "C" int mmsp_gpu_create(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc)
         cudaGetLastError();
         return MMSP_GPU_ENODEV;
     }
-    mmsp_gpu_handle* h = new (std::nothrow) mmsp_gpu_handle();
+    mmsp_gpu_handle* h = new_handle(desc);
     if (!h) return MMSP_GPU_ENOMEM;
-    memset(h, 0, sizeof(*h));
-    h->d = *desc;
-    for (int a = desc->dim; a < 3; a++) h->d.n[a] = 1;
-    h->g = pf::make_geom(h->d);
-    h->c = pf::make_coeffs(h->d);
-    cudaGetDevice(&h->device);
-    h->esize = esize_of(&h->d);
-    h->bytes = state_bytes(&h->d);
-    h->elems = h->bytes / h->esize;
-    cudaError_t e;
-    if ((e = cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking)) != cudaSuccess) goto cuda_err;
-    h->stream = h->own;
-    if ((e = cudaEventCreate(&h->ev0)) != cudaSuccess) goto cuda_err;
-    if ((e = cudaEventCreate(&h->ev1)) != cudaSuccess) goto cuda_err;
-    if (cudaMalloc(&h->buf[0], h->bytes) != cudaSuccess || cudaMalloc(&h->buf[1], h->bytes) != cudaSuccess ||
-        cudaMalloc((void**)&h->partials, pf::kPartialsBytes) != cudaSuccess ||
-        cudaMalloc((void**)&h->flags, 256) != cudaSuccess || cudaMemset(h->flags, 0, 256) != cudaSuccess ||
-        (work_bytes(&h->d) && cudaMalloc(&h->work, work_bytes(&h->d)) != cudaSuccess)) {
-        cudaGetLastError();
-        release(h);
+    Kit kit;
+    const cudaError_t e = take_kit(pf::handle_block_bytes(h->d), &kit);
+    if (e != cudaSuccess) {
         delete h;
-        return MMSP_GPU_ENOMEM;
+        return e == cudaErrorMemoryAllocation ? MMSP_GPU_ENOMEM : MMSP_GPU_ECUDA;
     }
-    rc = make_plan(h);
-    if (!rc) rc = setup_tb(h);
+    h->kit_ctx = kit.ctx;
+    h->kit_bytes = kit.bytes;
+    h->own = h->stream = kit.stream;
+    h->ev0 = kit.ev0;
+    h->ev1 = kit.ev1;
+    rc = set_up(h, kit.block);
     if (rc) {
         release(h);
         delete h;
@@ -475,18 +592,13 @@ extern "C" int mmsp_gpu_create(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc)
     }
     *out = h;
     return MMSP_GPU_OK;
-cuda_err:
-    release(h);
-    delete h;
-    cudaGetLastError();
-    return e == cudaErrorMemoryAllocation ? MMSP_GPU_ENOMEM : MMSP_GPU_ECUDA;
 }
 
 extern "C" int mmsp_gpu_destroy(mmsp_gpu_handle* h)
 {
     if (!h) return MMSP_GPU_OK;
-    cudaStreamSynchronize(h->stream);
-    release(h);
+    const bool idle = cudaStreamSynchronize(h->stream) == cudaSuccess;
+    release(h, idle);
     delete h;
     return MMSP_GPU_OK;
 }
@@ -550,7 +662,8 @@ static int upload(mmsp_gpu_handle* h, const void* src, size_t bytes, int layout,
     return MMSP_GPU_OK;
 }
 
-static int download(mmsp_gpu_handle* h, void* dst, size_t bytes, int layout, cudaMemcpyKind kind, bool sync)
+// `sync`: wait for the copy; `check`: report the status words too.
+static int download(mmsp_gpu_handle* h, void* dst, size_t bytes, int layout, cudaMemcpyKind kind, bool sync, bool check)
 {
     int rc = check_io(h, dst, bytes, layout);
     if (rc) return rc;
@@ -568,8 +681,9 @@ static int download(mmsp_gpu_handle* h, void* dst, size_t bytes, int layout, cud
     }
     e = cudaMemcpyAsync(dst, src, bytes, kind, h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "download");
+    if (check) return check_flags(h);
     if (sync && (e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return cuda_fail(h, e, "download sync");
-    return sync ? check_flags(h) : MMSP_GPU_OK;
+    return MMSP_GPU_OK;
 }
 
 extern "C" int mmsp_gpu_upload(mmsp_gpu_handle* h, const void* host, size_t bytes, int layout)
@@ -578,7 +692,7 @@ extern "C" int mmsp_gpu_upload(mmsp_gpu_handle* h, const void* host, size_t byte
 }
 extern "C" int mmsp_gpu_download(mmsp_gpu_handle* h, void* host, size_t bytes, int layout)
 {
-    return download(h, host, bytes, layout, cudaMemcpyDeviceToHost, true);
+    return download(h, host, bytes, layout, cudaMemcpyDeviceToHost, true, true);
 }
 extern "C" int mmsp_gpu_upload_device(mmsp_gpu_handle* h, const void* dev, size_t bytes, int layout)
 {
@@ -586,7 +700,7 @@ extern "C" int mmsp_gpu_upload_device(mmsp_gpu_handle* h, const void* dev, size_
 }
 extern "C" int mmsp_gpu_download_device(mmsp_gpu_handle* h, void* dev, size_t bytes, int layout)
 {
-    return download(h, dev, bytes, layout, cudaMemcpyDeviceToDevice, false);
+    return download(h, dev, bytes, layout, cudaMemcpyDeviceToDevice, false, false);
 }
 
 // One step on `s`.  The stochastic forms read the index of their noise
@@ -761,15 +875,21 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
     return MMSP_GPU_OK;
 }
 
-// After a synchronisation: report (and clear) a kernel's timed-out wait
+// Wait for the handle's work, then report (and clear) a kernel's timed-out wait
 // (word 0) or a sparse list that outgrew its slots (word 1).
 static int check_flags(mmsp_gpu_handle* h)
 {
     int f[2] = {0, 0};
-    cudaError_t e = cudaMemcpy(f, h->flags, sizeof(f), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(h, e, "flags");
+    cudaError_t e = cudaMemcpyAsync(f, h->flags, sizeof(f), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return cuda_fail(h, e, "synchronize");
+    return report_flags(h, f);
+}
+
+static int report_flags(mmsp_gpu_handle* h, const int* f)
+{
     if (f[0] || f[1]) {
-        cudaMemset(h->flags, 0, sizeof(f));
+        cudaMemset(h->flags, 0, 2 * sizeof(int));
         if (h->multi) {   // a launch that left early leaves its barrier word anywhere
             cudaMemset(multi_word(h), 0, sizeof(unsigned));
             h->multi_base = 0;
@@ -784,8 +904,6 @@ static int check_flags(mmsp_gpu_handle* h)
 extern "C" int mmsp_gpu_synchronize(mmsp_gpu_handle* h)
 {
     if (!h) return MMSP_GPU_EINVAL;
-    cudaError_t e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return cuda_fail(h, e, "synchronize");
     return check_flags(h);
 }
 
@@ -796,11 +914,17 @@ extern "C" int mmsp_gpu_reduce(mmsp_gpu_handle* h, mmsp_gpu_stats* st)
         return fail(h, MMSP_GPU_EUNSUPPORTED, "%s", "no reductions of sparse grids (the example reports none)");
     cudaError_t e = pf::launch_reduce(h->d, h->g, h->c, h->buf[h->cur], h->partials, h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "reduce");
-    double res[2];
-    e = cudaMemcpyAsync(res, h->partials + 4 * pf::kReduceBlocks, sizeof(res), cudaMemcpyDeviceToHost, h->stream);
+    // the results and, behind them, the status words in one copy
+    constexpr size_t at = 4 * pf::kReduceBlocks * sizeof(double), flags_at = (pf::kPartialsBytes + 255) / 256 * 256;
+    char both[flags_at - at + 2 * sizeof(int)];
+    e = cudaMemcpyAsync(both, h->partials + 4 * pf::kReduceBlocks, sizeof(both), cudaMemcpyDeviceToHost, h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "reduce copy");
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return cuda_fail(h, e, "reduce sync");
-    int rc = check_flags(h);
+    double res[2];
+    int f[2];
+    memcpy(res, both, sizeof(res));
+    memcpy(f, both + (flags_at - at), sizeof(f));
+    int rc = report_flags(h, f);
     if (rc) return rc;
     st->mass = res[0];
     st->energy = res[1];
@@ -832,10 +956,10 @@ extern "C" int mmsp_gpu_update(const mmsp_gpu_desc* desc, void* host, size_t byt
     mmsp_gpu_handle* h = nullptr;
     int rc = mmsp_gpu_create(&h, desc);
     if (rc) return rc;
-    rc = mmsp_gpu_upload(h, host, bytes, layout);
+    rc = upload(h, host, bytes, layout, cudaMemcpyHostToDevice, false);
     if (!rc) rc = mmsp_gpu_step(h, steps);
-    if (!rc && stats) rc = mmsp_gpu_reduce(h, stats);
-    if (!rc) rc = mmsp_gpu_download(h, host, bytes, layout);
+    if (!rc && stats) rc = mmsp_gpu_reduce(h, stats);   // reports the status words of the steps
+    if (!rc) rc = download(h, host, bytes, layout, cudaMemcpyDeviceToHost, true, !stats);
     mmsp_gpu_destroy(h);
     return rc;
 }

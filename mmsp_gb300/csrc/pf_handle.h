@@ -40,6 +40,8 @@ struct mmsp_gpu_handle {
     cudaStream_t own;        // private stream
     cudaStream_t stream;     // stream in use
     cudaEvent_t ev0, ev1;
+    unsigned long long kit_ctx;   // the set that own, ev0, ev1 and the block belong to (mmsp_gpu.cu)
+    size_t kit_bytes;
     bool timed;              // ev0/ev1 bracket the last step call
     bool external;           // buffers and stream belong to the caller (pf::create_in): not freed here
     int64_t steps;
