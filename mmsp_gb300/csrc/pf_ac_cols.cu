@@ -127,7 +127,11 @@ constexpr int cols_min_blocks()
     return V == 4 || N <= 8 ? 3 : V == 1 && N <= 16 ? 5 : N <= 16 ? 4 : 3;
 }
 
-template <int N, int V, int MODEL>
+// PRE: ask L2 for the cells of plane x+2 while plane x is worked on.  Only few
+// rolled values leave registers for several fields' loads in flight, and only
+// a dozen warps share an SM; the loads of plane x+1 then find L2 instead of
+// waiting for HBM.
+template <int N, int V, int MODEL, bool PRE>
 __global__ void __launch_bounds__(kAcColThreads, cols_min_blocks<N, V>())
 ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcColF32 q, int planes, int flip)
 {
@@ -165,6 +169,11 @@ ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcC
         const char* pc = in + x * pb;
         const char* ph = in + (x + 1 == g.X ? 0 : x + 1) * pb;
         char* po = out + x * pb;
+        if (PRE) {
+            const char* pn = in + (x + 2 >= g.X ? (x + 2) % g.X : x + 2) * pb;
+#pragma unroll
+            for (int f = 0; f < N; f++) asm volatile("prefetch.global.L2 [%0];" ::"l"(pn + f * fb + o));
+        }
         float sum[V];
 #pragma unroll
         for (int k = 0; k < V; k++) {
@@ -284,14 +293,28 @@ ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> pc0, i
 
 namespace {
 
-template <int N, int V>
+template <int N, int V, bool PRE>
 const void* cols_model(int model)
 {
-    if (model == MMSP_GPU_AC) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_AC>;
-    if (model == MMSP_GPU_GG) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_GG>;
-    if (model == MMSP_GPU_ZENER) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_ZENER>;
-    if (N == 1 && model == MMSP_GPU_AC_POLY) return (const void*)&ac_cols_f32<1, V, MMSP_GPU_AC_POLY>;
+    if (model == MMSP_GPU_AC) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_AC, PRE>;
+    if (model == MMSP_GPU_GG) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_GG, PRE>;
+    if (model == MMSP_GPU_ZENER) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_ZENER, PRE>;
+    if (N == 1 && model == MMSP_GPU_AC_POLY) return (const void*)&ac_cols_f32<1, V, MMSP_GPU_AC_POLY, PRE>;
     return nullptr;
+}
+
+// Prefetch (us per step without / with): V = 4 with 6 and 7 fields always,
+// 128^3 x 6 22.3 / 18.8, x 7 24.8 / 22.7, 80^3 x 6 8.3 / 8.3; 4 and 5 fields
+// never, 160^3 x 4 24.7 / 26.7, 148^3 x 5 25.8 / 26.7.  V = 1 with 5 to 9 fields
+// where the states exceed L2, 127^3 x 6 35.0 / 25.5, x 8 36.9 / 34.8, but 91^3
+// x 7 (42 MB) 12.4 / 13.1 and 127^3 x 10 43.4 / 45.3.  V = 2 never, 128^3 x 8
+// 24.1 / 26.0, 126^3 x 12 44.2 / 45.2.
+template <int N, int V>
+const void* cols_pre(int model, bool big)
+{
+    if constexpr (V == 4) return cols_model<N, V, (N >= 6)>(model);
+    else if constexpr (V == 1 && N >= 5 && N <= 9) return big ? cols_model<N, V, true>(model) : cols_model<N, V, false>(model);
+    else return cols_model<N, V, false>(model);
 }
 
 // V cells per thread, by the row length and the field count: vectors need
@@ -300,19 +323,21 @@ const void* cols_model(int model)
 // Measured, us per step: 128^3 x 7: 21.7 (V = 4), 31.9 (2), 31.6 (1); x 8:
 // 27.5 / 24.5 / 36.9; x 16: 62 / 55 / 85; 74^3 x 14: 10.3 (V = 2), 12.4 (1).
 template <int V, int LO, int HI>
-const void* cols_fn(int n, int model)
+const void* cols_fn(int n, int model, bool big)
 {
     if constexpr (LO > HI) {
         return nullptr;
     } else {
-        return n == LO ? cols_model<LO, V>(model) : cols_fn<V, LO + 1, HI>(n, model);
+        return n == LO ? cols_pre<LO, V>(model, big) : cols_fn<V, LO + 1, HI>(n, model, big);
     }
 }
 
-const void* cols_pick(int Z, int n, int model, int* v)
+const void* cols_pick(int Z, int n, int model, bool big, int* v)
 {
     *v = Z % 4 == 0 && n <= 7 ? 4 : Z % 2 == 0 && n <= 16 ? 2 : 1;
-    return *v == 4 ? cols_fn<4, 1, 7>(n, model) : *v == 2 ? cols_fn<2, 1, 16>(n, model) : cols_fn<1, 1, 32>(n, model);
+    return *v == 4   ? cols_fn<4, 1, 7>(n, model, big)
+           : *v == 2 ? cols_fn<2, 1, 16>(n, model, big)
+                     : cols_fn<1, 1, 32>(n, model, big);
 }
 
 template <typename T, int DIM, bool UNIT>
@@ -370,16 +395,16 @@ cudaError_t plan_ac(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
         p->ok = true;
         return cudaSuccess;
     }
+    const bool big = 2LL * g.cells * d.fields * (long long)sizeof(float) > kAcColL2;
     int v = 1;
-    p->fn = cols_pick(g.Z, d.fields, d.model, &v);
+    p->fn = cols_pick(g.Z, d.fields, d.model, big, &v);
     if (!p->fn) return cudaErrorInvalidConfiguration;
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->fn, kAcColThreads, 0);
     if (e != cudaSuccess) return e;
     const long long cols = (g.YZ / v + kAcColThreads - 1) / kAcColThreads;
     const long long slots = (long long)sm_count() * std::max(1, per_sm);
-    long long planes = 2LL * g.cells * d.fields * (long long)sizeof(float) > kAcColL2 ? (d.fields <= 8 ? 3 : 2)
-                                                                                     : (cols * g.X + slots - 1) / slots;
+    long long planes = big ? (d.fields <= 8 ? 3 : 2) : (cols * g.X + slots - 1) / slots;
     planes = std::max(planes, (long long)(g.X + 65534) / 65535);
     planes = std::min(std::max(planes, 1LL), (long long)g.X);
     p->planes = (int)planes;

@@ -68,3 +68,24 @@ def test_column_kernel_above_l2(gpu, oracle, shape, fields):
         s.step(3)
         got = s.download().astype(np.float64)
     assert np.abs(got - oracle.ac_baseline(x, 3, 1.5, 2.0, 1.0, 0.05)).max() <= TOL_F32
+
+
+# the form that prefetches a plane ahead: odd rows, 5 to 9 fields, above 96 MB;
+# fewer planes than a run, a run and one plane, several runs
+@pytest.mark.parametrize("shape,fields,model", [((2, 2521, 501), 5, "ac"), ((4, 1181, 333), 9, "gg"),
+                                                ((19, 250, 333), 8, "zener")])
+def test_prefetching_column_kernel(gpu, oracle, shape, fields, model):
+    from mmsp_gb300 import inputs
+
+    x = inputs.voronoi_grains(shape, 5, fields, 78) * 0.8 + 0.05
+    if model == "ac":
+        d = gpu.make_desc(shape, fields, np.float32, "ac", gamma=1.5, kappa=2.0, mobility=1.0, dt=0.05)
+        want = oracle.ac_baseline(x, 3, 1.5, 2.0, 1.0, 0.05)
+    else:
+        d = gpu.make_desc(shape, fields, np.float32, model, dt=0.01)
+        want = (oracle.ac_graingrowth if model == "gg" else oracle.ac_zener)(x, 3, 0.01)
+    with gpu.Stepper(d) as s:
+        s.upload(x.astype(np.float32))
+        s.step(3)
+        got = s.download().astype(np.float64)
+    assert np.abs(got - want).max() <= TOL_F32
