@@ -19,8 +19,18 @@ using pf::Coeffs;
 using pf::Geom;
 using pf::StepPlan;
 
-static const int kGraphSteps = 64;
-static const int kGraphMin = 2 * kGraphSteps;   // replay only for runs this long
+// Runs of kGraphLongMin launches and more replay a CUDA graph of
+// kGraphLaunches[1] launches, shorter ones and remainders of kGraphMin and more
+// one of kGraphLaunches[0] (even counts: a replay ends in the buffer that it
+// began in).  A launch of a graph follows the one before it 2 us sooner than a
+// launch on a stream, or than the first of the next replay; making a graph costs
+// about 3 us a launch, once per handle.  us per step, 40^3 FP32 Cahn-Hilliard,
+// launches on the stream / a handle's first call with the short graph / later
+// calls: 32 steps 5.56 / 5.08 / 3.54, 64 steps 5.3 / 3.9 / 3.15, 100 steps 5.2 /
+// 3.7 / 3.2.  74^3 x 14 Allen-Cahn, 200 steps a call: 10.8 with the short graph,
+// 10.7 with the long one; graphs of 8 cost 5% over those of 64.
+static const int kGraphLaunches[2] = {16, 64};
+static const int kGraphMin = 32, kGraphLongMin = 192;
 
 static int fail(mmsp_gpu_handle* h, int code, const char* fmt, const char* a = "", const char* b = "")
 {
@@ -380,7 +390,8 @@ static void give_kit(Kit kit, bool idle)
 static void release(mmsp_gpu_handle* h, bool idle = false)
 {
     if (h->out) pf::output_release(h);   // waits for snapshots still being written
-    if (h->graph) cudaGraphExecDestroy(h->graph);
+    for (cudaGraphExec_t g : h->graph)
+        if (g) cudaGraphExecDestroy(g);
     if (h->external) {   // the caller's block and stream
         if (h->ev0) cudaEventDestroy(h->ev0);
         if (h->ev1) cudaEventDestroy(h->ev1);
@@ -722,9 +733,14 @@ static cudaError_t one_step(mmsp_gpu_handle* h, cudaStream_t s)
     return e;
 }
 
-static int build_graph(mmsp_gpu_handle* h)
+// One launch of a blocked handle (kTbAnyDepth steps), else one step.
+static cudaError_t one_launch(mmsp_gpu_handle* h, cudaStream_t s) { return h->tb ? tb_launch(h, s) : one_step(h, s); }
+
+// The graph of kGraphLaunches[which] launches from buf[0], at an even launch
+// count of the blocked kernel.
+static int build_graph(mmsp_gpu_handle* h, int which)
 {
-    if (h->graph) return MMSP_GPU_OK;   // kernel nodes do not depend on the launch stream
+    if (h->graph[which]) return MMSP_GPU_OK;   // kernel nodes do not depend on the launch stream
     // capture on a private stream so a caller's legacy/default stream works too
     cudaStream_t cs;
     cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
@@ -739,10 +755,7 @@ static int build_graph(mmsp_gpu_handle* h)
     h->cur = 0;
     h->tb_launches = 0;
     cudaError_t le = cudaSuccess;
-    if (h->tb)
-        for (int i = 0; i < kGraphSteps / pf::kTbAnyDepth && le == cudaSuccess; i++) le = tb_launch(h, cs);
-    else
-        for (int i = 0; i < kGraphSteps && le == cudaSuccess; i++) le = one_step(h, cs);
+    for (int i = 0; i < kGraphLaunches[which] && le == cudaSuccess; i++) le = one_launch(h, cs);
     h->cur = saved;
     h->tb_launches = saved_launches;
     cudaGraph_t graph = nullptr;
@@ -752,12 +765,43 @@ static int build_graph(mmsp_gpu_handle* h)
         if (graph) cudaGraphDestroy(graph);
         return cuda_fail(h, le != cudaSuccess ? le : e, "capture");
     }
-    e = cudaGraphInstantiate(&h->graph, graph, 0);
+    e = cudaGraphInstantiate(&h->graph[which], graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
-        h->graph = nullptr;
+        h->graph[which] = nullptr;
         return cuda_fail(h, e, "instantiate");
     }
+    return MMSP_GPU_OK;
+}
+
+// `left` launches on the handle's stream.
+static int run_launches(mmsp_gpu_handle* h, int left)
+{
+    cudaError_t e;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (left >= kGraphMin && (e = cudaStreamIsCapturing(h->stream, &capture)) != cudaSuccess)
+        return cuda_fail(h, e, "step");
+    // a caller who captures the stream gets the launches themselves
+    if (left >= kGraphMin && capture == cudaStreamCaptureStatusNone) {
+        // the tile kernel's work counter follows the launch count, which must be even too
+        auto off = [&] { return h->tb && !h->tb_strips ? (int)(h->tb_launches & 1) : h->cur; };
+        if (h->cur == 1 && off()) {
+            if ((e = one_launch(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "step");
+            left--;
+        }
+        for (int which = left >= kGraphLongMin ? 1 : 0; which >= 0 && h->cur == 0 && !off(); which--) {
+            if (left < kGraphMin) break;
+            const int n = kGraphLaunches[which], rc = build_graph(h, which);
+            if (rc) return rc;
+            for (; left >= n; left -= n) {
+                if ((e = cudaGraphLaunch(h->graph[which], h->stream)) != cudaSuccess)
+                    return cuda_fail(h, e, "graph launch");
+                if (h->tb) h->tb_launches += n;
+            }
+        }
+    }
+    for (; left > 0; left--)
+        if ((e = one_launch(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "step");
     return MMSP_GPU_OK;
 }
 
@@ -830,45 +874,13 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
         int rc = convex_steps(h, steps);
         if (rc) return rc;
         left = 0;
-    } else if (h->tb) {
-        constexpr int kTbGraph = kGraphSteps / pf::kTbAnyDepth;   // launches per graph replay (even)
-        int nt = left / pf::kTbAnyDepth;
-        left -= nt * pf::kTbAnyDepth;
-        if (nt >= 2 * kTbGraph) {
-            int rc = build_graph(h);
-            if (rc) return rc;
-            // the graph starts from buf[0] at an even launch count
-            if (h->cur == 1 && (h->tb_launches & 1) == 1) {
-                if ((e = tb_launch(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "blocked step");
-                nt--;
-            }
-            if (h->cur == 0 && (h->tb_launches & 1) == 0)
-                while (nt >= kTbGraph) {
-                    if ((e = cudaGraphLaunch(h->graph, h->stream)) != cudaSuccess) return cuda_fail(h, e, "graph launch");
-                    nt -= kTbGraph;
-                    h->tb_launches += kTbGraph;
-                }
-        }
-        while (nt > 0) {
-            if ((e = tb_launch(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "blocked step");
-            nt--;
-        }
-    } else if (steps >= kGraphMin) {
-        int rc = build_graph(h);
+    } else {
+        const int rc = run_launches(h, h->tb ? left / pf::kTbAnyDepth : left);
         if (rc) return rc;
-        if (h->cur == 1) {
-            if ((e = one_step(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "step");
-            left--;
-        }
-        while (left >= kGraphSteps) {
-            if ((e = cudaGraphLaunch(h->graph, h->stream)) != cudaSuccess) return cuda_fail(h, e, "graph launch");
-            left -= kGraphSteps;   // even count: the state is back in buf[0]
-        }
+        left = h->tb ? left % pf::kTbAnyDepth : 0;   // a blocked handle's last steps
     }
-    while (left > 0) {
+    for (; left > 0; left--)
         if ((e = one_step(h, h->stream)) != cudaSuccess) return cuda_fail(h, e, "step");
-        left--;
-    }
     if ((e = cudaEventRecord(h->ev1, h->stream)) != cudaSuccess) return cuda_fail(h, e, "event");
     h->timed = true;
     h->steps += steps;

@@ -45,9 +45,9 @@ struct mmsp_gpu_handle {
     bool timed;              // ev0/ev1 bracket the last step call
     bool external;           // buffers and stream belong to the caller (pf::create_in): not freed here
     int64_t steps;
-    // CUDA graph of kGraphSteps steps starting from buf[0] (an even count ends in buf[0]); for
-    // blocked handles, kGraphSteps / pf::kTbAnyDepth launches from buf[0] at an even launch count
-    cudaGraphExec_t graph;
+    // CUDA graphs of a short and a long run of launches from buf[0] (at an even launch count of the
+    // blocked kernel), ending in buf[0]
+    cudaGraphExec_t graph[2];
     pf::OutputState* out;    // snapshot writer (mmsp_gpu_output), created on first use
     unsigned last_iters;     // MMSP_GPU_CH_CONVEX: solver iterations of the last step
     // small 2D FP64 Cahn-Hilliard: many steps per cooperative launch; the value of its barrier word
