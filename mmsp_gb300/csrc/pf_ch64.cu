@@ -80,6 +80,19 @@ static __device__ __forceinline__ double nsum(const Ar<double>& A, double sx, do
     return DIM == 3 ? fma(q.wx, sx, fma(q.wy, sy, A.mul(q.wz, sz))) : fma(q.wy, sy, A.mul(q.wz, sz));
 }
 
+// Contracted mu from the neighbours' sum: f'(c) - kappa (S - w2 c) = c * (poly0 + ...) - kappa S
+template <int MODEL, bool KONE>
+static __device__ __forceinline__ double mu_sum(const Ar<double>& A, double c, double s, const C64& q)
+{
+    double t;
+    if (MODEL == MMSP_GPU_CH) {   // 2c(1-c)(1-2c) = c (2 + c (-6 + 4c))
+        t = fma(fma(q.four, c, -q.six), c, q.poly0);
+    } else {                      // -r c + u c^3 = c (-r + u c^2)
+        t = fma(q.u, A.mul(c, c), q.poly0);
+    }
+    return KONE ? fma(t, c, -s) : fma(-q.kappa, s, A.mul(t, c));
+}
+
 template <int DIM, int MODEL, bool UNIT, bool KONE, bool EXACT>
 static __device__ __forceinline__ double mu_cell(const Ar<double>& A, double c, double xh, double xl, double yh, double yl,
                                                  double zh, double zl, const C64& q, const P<double>& p)
@@ -91,15 +104,7 @@ static __device__ __forceinline__ double mu_cell(const Ar<double>& A, double c, 
         if (KONE) pk.kappa = 1.0;   // constant: kappa_times folds to lap
         return ch_mu<double, MODEL>(A, c, lap, pk);
     }
-    // mu = f'(c) - kappa (S - w2 c) = c * (poly0 + ...) - kappa S
-    const double s = nsum<DIM, UNIT>(A, A.add(xh, xl), A.add(yh, yl), A.add(zh, zl), q);
-    double t;
-    if (MODEL == MMSP_GPU_CH) {   // 2c(1-c)(1-2c) = c (2 + c (-6 + 4c))
-        t = fma(fma(q.four, c, -q.six), c, q.poly0);
-    } else {                      // -r c + u c^3 = c (-r + u c^2)
-        t = fma(q.u, A.mul(c, c), q.poly0);
-    }
-    return KONE ? fma(t, c, -s) : fma(-q.kappa, s, A.mul(t, c));
+    return mu_sum<MODEL, KONE>(A, c, nsum<DIM, UNIT>(A, A.add(xh, xl), A.add(yh, yl), A.add(zh, zl), q), q);
 }
 
 template <int DIM, int MODEL, bool UNIT, bool KONE, bool EXACT, bool NOISE>
@@ -178,6 +183,88 @@ ch64_update(const double* __restrict__ cin, const double* __restrict__ mu, doubl
         a = b;
         b = n;
     }
+}
+
+// Contracted form on unit spacing, 3D: the same two passes with fewer additions.
+//
+// With D(x, y) = f(x+1, y) + f(x, y+1), the four neighbours along X and Y of a
+// cell are D(x, y) + D(x-1, y-1): one addition a cell for D, one for the sum, in
+// place of three.  A thread owns kC64Rows rows and walks X, so D(x-1, y-1) is
+// the D of its row above from the plane before; only the first row's, and a
+// run's first plane's, are added up anew: a Laplacian takes 4 + 1/R + 1/planes
+// additions for 5, a step 14.3 operations for 15.  Bound by the FP64 pipe as the
+// two passes above.  256^3: 412 -> 395 us per step, 16.8 M * 14.3 / 395 us =
+// 0.61 T operations per second.  us per step by rows (planes of the best run):
+// 256^3 394 (2 rows, 8 planes), 392 (4, 8), 389 (6, 5), but 187^3 164 (2, 6),
+// 165 (4, 4), 165 (6, 4) and 160^3 103 (2, 6), 104 (4, 3), 103 (6, 3): more rows
+// want a length of run for each grid, so that no SM gets a block more than the
+// others.  One warp a block: those blocks are the smallest.
+constexpr int kC64Rows = 2, kC64PairPlanes = 6;
+constexpr long long kC64PairCells = 1LL << 22;
+
+template <typename F>
+static __device__ __forceinline__ void walk_pairs(const Ar<double>& A, const double* __restrict__ f, const Geom& g,
+                                                  int planes, F out)
+{
+    constexpr int R = kC64Rows;
+    const int z = blockIdx.x * kC64Z + threadIdx.x;
+    if (z >= g.Z) return;   // no barrier
+    const int y0 = min((int)blockIdx.y * R, g.Y - R);   // the last strip may repeat a row of the one before
+    const int dzl = z == 0 ? g.Z - 1 : -1, dzh = z + 1 == g.Z ? -z : 1;
+    const long long row = (long long)y0 * g.Z + z;
+    const long long rl = (long long)(y0 == 0 ? g.Y - 1 : y0 - 1) * g.Z + z;
+    const long long rh = (long long)(y0 + R == g.Y ? 0 : y0 + R) * g.Z + z;
+    const int xs = blockIdx.z * planes, xe = min(xs + planes, g.X);
+    double c[R + 1], d[R];   // plane x on rows y0 .. y0+R; D(x-1, y-1) on rows y0 .. y0+R-1
+    {
+        const double* pl = f + (long long)(xs == 0 ? g.X - 1 : xs - 1) * g.YZ;
+        const double* pc = f + (long long)xs * g.YZ;
+#pragma unroll
+        for (int r = 0; r < R; r++) c[r] = __ldg(pc + row + (long long)r * g.Z);
+        c[R] = __ldg(pc + rh);
+#pragma unroll
+        for (int r = 0; r < R; r++) d[r] = A.add(r == 0 ? __ldg(pc + rl) : c[r - 1], __ldg(pl + row + (long long)r * g.Z));
+    }
+    for (int x = xs; x < xe; x++) {
+        const double* pc = f + (long long)x * g.YZ + row;
+        const double* ph = f + (long long)(x + 1 == g.X ? 0 : x + 1) * g.YZ;
+        double n[R + 1], e[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) n[r] = __ldg(ph + row + (long long)r * g.Z);
+        n[R] = __ldg(ph + rh);
+        const double nl = __ldg(ph + rl);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const double* pz = pc + (long long)r * g.Z;
+            const double sz = A.add(__ldg(pz + dzh), __ldg(pz + dzl));
+            e[r] = A.add(n[r], c[r + 1]);
+            out((long long)x * g.YZ + row + (long long)r * g.Z, c[r], A.add(A.add(e[r], d[r]), sz));
+        }
+        d[0] = A.add(nl, c[0]);
+#pragma unroll
+        for (int r = 1; r < R; r++) d[r] = e[r - 1];
+#pragma unroll
+        for (int r = 0; r <= R; r++) c[r] = n[r];
+    }
+}
+
+template <int MODEL, bool KONE>
+__global__ void __launch_bounds__(kC64Z)
+ch64_mu_pairs(const double* __restrict__ cin, double* __restrict__ mu, Geom g, C64 q0, P<double>, int planes)
+{
+    const Ar<double> A(g.dim);
+    const C64 q = held(A, q0);
+    walk_pairs(A, cin, g, planes, [&](long long i, double c, double s) { mu[i] = mu_sum<MODEL, KONE>(A, c, s, q); });
+}
+
+__global__ void __launch_bounds__(kC64Z)
+ch64_update_pairs(const double* __restrict__ cin, const double* __restrict__ mu, double* __restrict__ cout, Geom g, C64 q0,
+                  P<double>, int planes)
+{
+    const Ar<double> A(g.dim);
+    const C64 q = held(A, q0);
+    walk_pairs(A, mu, g, planes,
+               [&](long long i, double m, double s) { cout[i] = fma(q.dtm, s, fma(q.upd0, m, __ldg(cin + i))); });
 }
 
 // Small 2D grids: many steps in one cooperative launch.  The two passes above
@@ -480,10 +567,24 @@ cudaError_t plan_ch64(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
                            : mu_fn_m<2>(d.model, c.unit_w, kone, exact, noise);
         p->fn2 = g.dim == 3 ? upd_fn<3>(c.unit_w, exact) : upd_fn<2>(c.unit_w, exact);
     }
-    p->block = dim3(kC64Z, kC64Y, 1);
     p->planes = g.dim == 3 ? kC64Planes : 1;
+    unsigned warps_y = kC64Y, rows = 1;
+    // Fewer additions a cell, but threads with more to do: 256^3 412 -> 395 us
+    // per step, 224^3 278 -> 269, 187^3 168 -> 164, 160^3 104.5 -> 102.8; but 128^3 55 -> 58.
+    if (d.dtype == MMSP_GPU_F64 && g.dim == 3 && !exact && !noise && c.unit_w && g.cells >= kC64PairCells &&
+        g.Y >= kC64Rows && g.Y <= 65535 * kC64Rows) {
+        p->fn = d.model == MMSP_GPU_CH ? (kone ? (const void*)&ch64_mu_pairs<MMSP_GPU_CH, true>
+                                               : (const void*)&ch64_mu_pairs<MMSP_GPU_CH, false>)
+                                       : (kone ? (const void*)&ch64_mu_pairs<MMSP_GPU_CH_POLY, true>
+                                               : (const void*)&ch64_mu_pairs<MMSP_GPU_CH_POLY, false>);
+        p->fn2 = (const void*)&ch64_update_pairs;
+        p->planes = kC64PairPlanes;
+        warps_y = 1;
+        rows = kC64Rows;
+    }
+    p->block = dim3(kC64Z, warps_y, 1);
     const int segs = (g.X + p->planes - 1) / p->planes;
-    p->grid = dim3((g.Z + kC64Z - 1) / kC64Z, (g.Y + kC64Y - 1) / kC64Y, segs);
+    p->grid = dim3((g.Z + kC64Z - 1) / kC64Z, (g.Y + warps_y * rows - 1) / (warps_y * rows), segs);
     p->smem = 0;
     p->fields = 1;
     p->kind = 6;
