@@ -774,15 +774,12 @@ static int build_graph(mmsp_gpu_handle* h, int which)
     return MMSP_GPU_OK;
 }
 
-// `left` launches on the handle's stream.
-static int run_launches(mmsp_gpu_handle* h, int left)
+// `left` launches on the handle's stream.  A caller who captures the stream gets
+// the launches themselves.
+static int run_launches(mmsp_gpu_handle* h, int left, bool captured)
 {
     cudaError_t e;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (left >= kGraphMin && (e = cudaStreamIsCapturing(h->stream, &capture)) != cudaSuccess)
-        return cuda_fail(h, e, "step");
-    // a caller who captures the stream gets the launches themselves
-    if (left >= kGraphMin && capture == cudaStreamCaptureStatusNone) {
+    if (left >= kGraphMin && !captured) {
         // the tile kernel's work counter follows the launch count, which must be even too
         auto off = [&] { return h->tb && !h->tb_strips ? (int)(h->tb_launches & 1) : h->cur; };
         if (h->cur == 1 && off()) {
@@ -859,8 +856,12 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
         e = cudaMemsetAsync(h->buf[h->cur ^ 1], 0, sizeof(int) * (size_t)h->g.cells, h->stream);
         if (e != cudaSuccess) return cuda_fail(h, e, "sparse newGrid");
     }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if ((e = cudaStreamIsCapturing(h->stream, &capture)) != cudaSuccess) return cuda_fail(h, e, "step");
+    const bool captured = capture != cudaStreamCaptureStatusNone;
     int left = steps;
-    if (h->multi) {
+    // (a replay of a captured many-steps launch would wait for barrier counts of the past)
+    if (h->multi && !captured) {
         while (left > 0) {
             const int n = std::min(left, kMultiSteps);
             e = pf::launch_ch64_steps(h->ch64s, h->d, h->g, h->c, h->buf[h->cur], h->buf[h->cur ^ 1], n, multi_word(h),
@@ -875,7 +876,7 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
         if (rc) return rc;
         left = 0;
     } else {
-        const int rc = run_launches(h, h->tb ? left / pf::kTbAnyDepth : left);
+        const int rc = run_launches(h, h->tb ? left / pf::kTbAnyDepth : left, captured);
         if (rc) return rc;
         left = h->tb ? left % pf::kTbAnyDepth : 0;   // a blocked handle's last steps
     }

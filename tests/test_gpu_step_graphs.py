@@ -36,11 +36,13 @@ def test_one_call_equals_short_calls(gpu, shape, fields, dtype, model, per, lead
             assert np.array_equal(a.download(), b.download()), n
 
 
-def test_steps_on_a_captured_stream(gpu):
+@pytest.mark.parametrize("shape,dtype", [((20, 24, 28), np.float32), ((48, 50), np.float64), ((48, 50), np.float32)],
+                         ids=["3d-f32", "2d-f64", "2d-f32"])
+def test_steps_on_a_captured_stream(gpu, shape, dtype):
     import torch
 
-    d = gpu.make_desc((20, 24, 28), 1, np.float32, "ch", dt=0.002)
-    x = state((20, 24, 28), 1, np.float32)
+    d = gpu.make_desc(shape, 1, dtype, "ch", dt=0.002)
+    x = state(shape, 1, dtype)
     stream = torch.cuda.Stream()
     with gpu.Stepper(d) as s:
         s.upload(x)
