@@ -55,9 +55,11 @@ DT, KAPPA, MOB = 0.002, 1.0, 1.0
 MEAN, AMP, SEED = 0.4, 0.02, 2
 WORKLOAD = "ch3d_256_f64"
 # FP64 pipe operations (add, multiply or fused multiply-add) per cell-step of
-# the two FP64 forms (pf_ch64.cu: 9 + 7 contracted, 13 + 10 exact)
-F64_OPS_CONTRACT = 16
+# the two FP64 forms at 256^3 (pf_ch64.cu: contracted 7.67 + 6.67, a Laplacian's
+# pair sums shared by runs of 2 rows and 6 planes; exact 13 + 10)
+F64_OPS_CONTRACT = 43.0 / 3.0
 F64_OPS_EXACT = 23
+TILE_ROWS = (64, 96, 128)   # region rows of the tile kernel of the batched form; the strip kernel has others
 
 
 def dist_env():
@@ -574,8 +576,8 @@ def run_gpu(args):
                          "newGrid, temp)"},
         "roofline": {"bound": "fp64", "achieved": fp64_achieved / 1e12, "peak": fp64_peak / 1e12,
                      "unit": "T FP64 ops/s", "frac": fp64_achieved / fp64_peak,
-                     "traffic": profile_traffic("ch64_step_f64_256"),
-                     "kernel": "ch64_mu + ch64_update (one step: two launches)",
+                     "traffic": profile_traffic("ch64_pairs_f64_256"),
+                     "kernel": "ch64_mu_pairs + ch64_update_pairs (one step: two launches)",
                      "peak_source": "measured live: mmsp_gpu_fp64_rate (independent FP64 FMA chains, all SMs)",
                      "ops_per_launch": F64_OPS_CONTRACT * cells, "ops_per_cell": F64_OPS_CONTRACT,
                      "hbm": {"alg_bytes_per_step": cells * 40,
@@ -709,10 +711,12 @@ def batched(native, inputs, stream, reps, flush):
                               "temporal_depth": info.temporal_depth, "tile_rows": info.tile_rows,
                               "tile_cols": info.tile_cols, "tiles": info.tiles}},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": profile_traffic("ch2_tb_f32_256grids" if info.temporal_depth > 1
+                     "traffic": profile_traffic(("ch2_tb_f32_256grids" if info.tile_rows in TILE_ROWS
+                                                 else "ch2_strip_f32_256grids") if info.temporal_depth > 1
                                                 else "ch2_batch_f32_256grids"),
-                     "kernel": ("temporally blocked, CH, region %dx%d, KS=%d (%d steps per launch)" % (
-                         info.tile_rows, info.tile_cols, info.temporal_depth, info.temporal_depth)
+                     "kernel": ("%s<CH, unit>, region %dx%d (%d steps per launch)" % (
+                         "ch2_tb_kernel" if info.tile_rows in TILE_ROWS else "ch2_strip_kernel",
+                         info.tile_rows, info.tile_cols, info.temporal_depth)
                                 if info.temporal_depth > 1 else "ch2_batch_kernel<float,CH>"),
                      "peak_source": peak_kind, "alg_bytes_per_step": cells * 8,
                      "note": "achieved = the per-step algorithmic bytes (one read + one write of every cell) over the "
@@ -908,7 +912,7 @@ def run_case(name: str, steps: int):
         with native.Batch(descs) as b:
             for i, (c0, _) in enumerate(work):
                 b.upload(i, c0.astype(np.float32))
-            b.tune()          # 10 candidates x 4 launches before the measured steps
+            b.tune()          # its candidates' launches come before the measured steps
             b.step(steps)
             b.synchronize()
             inf = b.info()

@@ -12,7 +12,9 @@
 //   exact form       23 operations per cell (13 for mu, 10 for the update),
 //                    the reference's order, every operation rounded on its
 //                    own: bit-identical to the reference
-//   contracted form  16 operations per cell: the six-neighbour sum once,
+//   contracted form  15 operations per cell on unit spacing (14.3 with shared
+//                    pair sums, below; one more where kappa is not 1): the
+//                    six-neighbour sum once,
 //                    the centre term folded into the chemical potential's
 //                    polynomial and into the update's multiply-add.  Within
 //                    a few ulps per step of the exact form; held to 1e-12
