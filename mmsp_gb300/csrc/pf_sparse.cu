@@ -180,35 +180,49 @@ static __device__ __noinline__ void sparse_cell(SpView in, SpView out, Geom g, S
 //
 // Bound: the FP64 pipe (about 18 operations per cell and grain, and a warp
 // takes as many rounds as its busiest cell; 55% busy) and load latency.  us per
-// step, walking the lists in global memory for every value / here: 512x512
-// cells of 160 grains 78.5 / 55.1 (500 steps from one item per cell; 60 steps
+// step, walking the lists in global memory for every value / here with a row of
+// cells a warp: 512x512 cells of 160 grains 78.5 / 55.1 (500 steps from one item per cell; 60 steps
 // 55.5 / 41.8), 2048x2048 of 32 grains 201 / 154, 48^3 of 12 grains 100 / 58.
 // (A dense table of a tile's grains in shared memory, behind a hashed
 // dictionary, took 65, 64, 229 and 82: its set-up costs more than the walks.)
 // 64-thread blocks of at most 64 registers: with 128 threads 60.9, with 72
 // registers 58.6.
+// BAND: a warp's cells are a patch of the plane, BAND rows by 32 / BAND columns,
+// instead of 32 in a row: they lie closer together, so their numbers of grains
+// differ less.  us per step in a row / in bands of 2 / 4 / 8 rows: 512x512 54.9
+// / 50.6 / 48.5 / 49.4, 2048x2048 157 / 151 / 144 / 148, 48^3 55.8 / 51.8 / 50.1
+// / 51.3, 41^3 55.4 / 54.9 / 54.7 / 54.7; but 25^3 55.2 / 56.0 / 56.5 / 56.5 and
+// 33x50x27 42.0 / 42.4 / 42.5 / 42.7, one wave of blocks: small grids, and 1D,
+// keep the row (kSpBandCells).
 constexpr int kSpThreads = 64;
 constexpr int kSpUnion = 16;
 constexpr int kSpBatch = 4;   // items of a list that are loaded at once
+constexpr long long kSpBandCells = 1LL << 16;
 
-template <int DIM, bool UNIT>
+template <int DIM, bool UNIT, int BAND>
 __global__ void __launch_bounds__(kSpThreads, 16)
 sparse_gg_step(SpView in, SpView out, Geom g, SpConst q0, int K, int* __restrict__ err)
 {
     __shared__ int s_key[kSpUnion][kSpThreads];
     __shared__ unsigned long long s_pos[kSpUnion][kSpThreads];   // slot + 1 in list l at bit 6*l, 0: not there
     const int tid = threadIdx.x;
-    const long long c = (long long)blockIdx.x * kSpThreads + tid;
-    if (c >= g.cells) return;   // no barrier in this kernel
+    const long long k0 = (long long)blockIdx.x * kSpThreads + tid;
+    if (k0 >= g.cells) return;   // no barrier in this kernel
     const long long cells = g.cells;
+    // the cells of a plane in bands of BAND rows (the last may have fewer), down each column of a band in turn
+    const int x = (int)(k0 / g.YZ);
+    const int r = (int)(k0 - (long long)x * g.YZ);
+    int y = r / g.Z / BAND * BAND, z = r - y * g.Z;
+    if constexpr (BAND > 1) {
+        const int e = z, rows = min(BAND, g.Y - y);
+        z = rows == BAND ? e / BAND : e / rows;
+        y += e - z * rows;
+    }
+    const long long c = (long long)x * g.YZ + (long long)y * g.Z + z;
     // padded coordinates and the periodic face neighbours of the real axes,
     // in the reference's axis order (real axis 0 first); list 0 is the cell's
     // own, 1 + 2 ra and 2 + 2 ra the low and high neighbour's on axis ra, 7 the
     // destination's
-    const int x = (int)(c / g.YZ);
-    const int r = (int)(c - (long long)x * g.YZ);
-    const int y = r / g.Z;
-    const int z = r - y * g.Z;
     long long nb[1 + 2 * DIM];
     nb[0] = c;
     nb[2 * DIM - 1] = c + (z == 0 ? g.Z - 1 : -1);
@@ -363,6 +377,16 @@ __global__ void sparse_unpack(SpView d, int* __restrict__ hcnt, int* __restrict_
 
 static unsigned blocks_for(long long cells, int threads = 128) { return (unsigned)((cells + threads - 1) / threads); }
 
+template <int DIM>
+static const void* sparse_fn(bool unit, bool band)
+{
+    if constexpr (DIM > 1) {
+        if (band)
+            return unit ? (const void*)&sparse_gg_step<DIM, true, 4> : (const void*)&sparse_gg_step<DIM, false, 4>;
+    }
+    return unit ? (const void*)&sparse_gg_step<DIM, true, 1> : (const void*)&sparse_gg_step<DIM, false, 1>;
+}
+
 cudaError_t launch_sparse_gg(const mmsp_gpu_desc& d, const Geom& g, const Coeffs& c, const void* in, void* out,
                              int* err, cudaStream_t s)
 {
@@ -372,10 +396,10 @@ cudaError_t launch_sparse_gg(const mmsp_gpu_desc& d, const Geom& g, const Coeffs
     for (int a = 0; a < 3; a++) q.w[a] = a < d.dim ? c.w[a] : 1.0;
     q.eps = d.aux[0];
     q.p = narrow<double>(c, g.dim);
-    const void* fn;
-    if (g.dim == 3) fn = c.unit_w ? (const void*)&sparse_gg_step<3, true> : (const void*)&sparse_gg_step<3, false>;
-    else if (g.dim == 2) fn = c.unit_w ? (const void*)&sparse_gg_step<2, true> : (const void*)&sparse_gg_step<2, false>;
-    else fn = c.unit_w ? (const void*)&sparse_gg_step<1, true> : (const void*)&sparse_gg_step<1, false>;
+    const bool band = g.dim > 1 && g.cells >= kSpBandCells;
+    const void* fn = g.dim == 3   ? sparse_fn<3>(c.unit_w, band)
+                     : g.dim == 2 ? sparse_fn<2>(c.unit_w, band)
+                                  : sparse_fn<1>(c.unit_w, false);
     int* ovf = err + 1;
     void* args[] = {(void*)&vi, (void*)&vo, (void*)&g, (void*)&q, (void*)&K, (void*)&ovf};
     return cudaLaunchKernel(fn, dim3(blocks_for(g.cells, kSpThreads)), dim3(kSpThreads), args, 0, s);
