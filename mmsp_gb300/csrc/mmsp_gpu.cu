@@ -563,7 +563,7 @@ static cudaError_t tb_launch(mmsp_gpu_handle* h, cudaStream_t s)
     const void* in = h->buf[h->cur];
     void* out = h->buf[h->cur ^ 1];
     const cudaError_t e =
-        h->tb_strips ? pf::launch_strips(h->tb_fn, h->tb_inst, h->tb_strip_list, h->tb_items, in, out, s)
+        h->tb_strips ? pf::launch_strips(h->tb_fn, h->tb_inst, h->tb_strip_list, h->tb_items, in, out, nullptr, 0, s)
                      : pf::launch_tb(h->tb_fn, h->tb_blocks, pf::kTbShapes[0].nt, h->tb_smem, h->tb_inst, h->tb_list,
                                      h->tb_items, in, out, h->tb_counters, (int)(h->tb_launches & 1), s);
     h->cur ^= 1;

@@ -463,14 +463,16 @@ static int set_tb(mmsp_gpu_batch* b, int shape, int ks)
     return MMSP_GPU_OK;
 }
 
-// tune.ks steps of every grid from pool `in` to pool `out` in one launch.
+// tune.ks steps of every grid from pool `in` to pool `out` in one launch.  Every
+// launch of a batch, of whatever kernel, finds counter `launches & 1` at zero
+// and leaves the other at zero, so the kernels may follow each other in any order.
 static cudaError_t step_tb(mmsp_gpu_batch* b, cudaStream_t s, int in, int out)
 {
     const int parity = (int)(b->launches & 1);
     b->launches++;
     if (shape_strips(b->tune.shape))
         return launch_strips(strip_kernel(b->persistent_model, b->unit, true), b->d_insts, b->d_strips, b->tb_nitems,
-                             b->pool[in], b->pool[out], s);
+                             b->pool[in], b->pool[out], b->counters, parity, s);
     return launch_tb(tb_kernel(b->tune.shape, b->tune.ks, b->persistent_model, b->unit), b->tb_blocks,
                      kTbShapes[b->tune.shape].nt, tb_smem(b->tune.shape), b->d_insts, b->d_tb, b->tb_nitems,
                      b->pool[in], b->pool[out], b->counters, parity, s);

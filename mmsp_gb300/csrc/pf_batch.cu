@@ -536,8 +536,10 @@ struct StripStage {
 template <int MODEL, bool UNIT, bool ALIGNED>
 __global__ void __launch_bounds__(kStripThreads, 3)
 ch2_strip_kernel(const BatchInst* __restrict__ insts, const StripItem* __restrict__ items, int nitems,
-                 const float* __restrict__ in, float* __restrict__ out)
+                 const float* __restrict__ in, float* __restrict__ out, int* __restrict__ counters, int parity)
 {
+    // takes no work from the counters, but leaves the next launch's at zero as the kernels that do
+    if (counters && blockIdx.x == 0 && threadIdx.x == 0) counters[parity ^ 1] = 0;
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * kStripThreads + threadIdx.x) >> 5);
     if (w >= nitems) return;   // whole warps
@@ -679,10 +681,11 @@ int strip_rows(int n0, int n1)
 }
 
 cudaError_t launch_strips(const void* fn, const BatchInst* insts, const StripItem* items, int nitems, const void* in,
-                          void* out, cudaStream_t s)
+                          void* out, int* counters, int parity, cudaStream_t s)
 {
     constexpr int per = kStripThreads / 32;
-    void* args[] = {(void*)&insts, (void*)&items, (void*)&nitems, (void*)&in, (void*)&out};
+    void* args[] = {(void*)&insts, (void*)&items, (void*)&nitems, (void*)&in, (void*)&out, (void*)&counters,
+                    (void*)&parity};
     return cudaLaunchKernel(fn, dim3((nitems + per - 1) / per), dim3(kStripThreads), args, 0, s);
 }
 

@@ -85,8 +85,10 @@ void strip_items(int inst, int n0, int n1, int rows, std::vector<StripItem>* ite
 // (2 rows), 1.50 (4), 1.63 (6), 1.94 (16), the rule's 4; 829 x 829 2.58 (8), 2.11
 // (11), 2.33 (16), the rule's 11; 4096 x 4096 19.2 (16), 12.3 (64), the rule's 11.6.
 int strip_rows(int n0, int n1);
+// `counters`, `parity`: the work counters of the other kernels in the same
+// sequence of launches, and this launch's place in it; NULL: no such counters.
 cudaError_t launch_strips(const void* fn, const BatchInst* insts, const StripItem* items, int nitems, const void* in,
-                          void* out, cudaStream_t s);
+                          void* out, int* counters, int parity, cudaStream_t s);
 
 const void* batch_kernel(int dtype, int model, bool unit);
 cudaError_t launch_batch(const void* fn, int blocks, int threads, const BatchInst* insts, const BatchItem* items,
