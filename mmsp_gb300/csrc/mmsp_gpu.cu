@@ -774,12 +774,34 @@ static int build_graph(mmsp_gpu_handle* h, int which)
     return MMSP_GPU_OK;
 }
 
-// `left` launches on the handle's stream.  A caller who captures the stream gets
-// the launches themselves.
-static int run_launches(mmsp_gpu_handle* h, int left, bool captured)
+// `left` launches on a stream that its caller captures: the launches themselves,
+// to be replayed from any state.  The tile kernel's launches take turns with its
+// two work counters, whose state a replay would find as the work before left it:
+// the captured launches start from two cleared counters and leave two cleared
+// ones, so that neither their number nor whether they run at all matters to the
+// handle's count.
+static int run_captured(mmsp_gpu_handle* h, int left)
+{
+    const bool counted = left > 0 && h->tb && !h->tb_strips;
+    const int64_t saved_launches = h->tb_launches;
+    cudaError_t e = cudaSuccess;
+    if (counted) {
+        h->tb_launches = 0;
+        e = cudaMemsetAsync(h->tb_counters, 0, 2 * sizeof(int), h->stream);
+    }
+    for (; left > 0 && e == cudaSuccess; left--) e = one_launch(h, h->stream);
+    if (counted) {
+        h->tb_launches = saved_launches;
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->tb_counters, 0, 2 * sizeof(int), h->stream);
+    }
+    return e == cudaSuccess ? MMSP_GPU_OK : cuda_fail(h, e, "captured step");
+}
+
+// `left` launches on the handle's stream.
+static int run_launches(mmsp_gpu_handle* h, int left)
 {
     cudaError_t e;
-    if (left >= kGraphMin && !captured) {
+    if (left >= kGraphMin) {
         // the tile kernel's work counter follows the launch count, which must be even too
         auto off = [&] { return h->tb && !h->tb_strips ? (int)(h->tb_launches & 1) : h->cur; };
         if (h->cur == 1 && off()) {
@@ -876,7 +898,8 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
         if (rc) return rc;
         left = 0;
     } else {
-        const int rc = run_launches(h, h->tb ? left / pf::kTbAnyDepth : left, captured);
+        const int launches = h->tb ? left / pf::kTbAnyDepth : left;
+        const int rc = captured ? run_captured(h, launches) : run_launches(h, launches);
         if (rc) return rc;
         left = h->tb ? left % pf::kTbAnyDepth : 0;   // a blocked handle's last steps
     }
