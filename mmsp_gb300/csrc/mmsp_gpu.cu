@@ -925,11 +925,14 @@ static int check_flags(mmsp_gpu_handle* h)
 static int report_flags(mmsp_gpu_handle* h, const int* f)
 {
     if (f[0] || f[1]) {
-        cudaMemset(h->flags, 0, 2 * sizeof(int));
+        // on the handle's stream, ahead of whatever it gets next: the default stream, which this one does not
+        // wait for, may be busy with the program's own work
+        cudaError_t e = cudaMemsetAsync(h->flags, 0, 2 * sizeof(int), h->stream);
         if (h->multi) {   // a launch that left early leaves its barrier word anywhere
-            cudaMemset(multi_word(h), 0, sizeof(unsigned));
+            if (e == cudaSuccess) e = cudaMemsetAsync(multi_word(h), 0, sizeof(unsigned), h->stream);
             h->multi_base = 0;
         }
+        if (e != cudaSuccess) return cuda_fail(h, e, "status words");
         if (f[0]) return fail(h, MMSP_GPU_ETIMEDOUT, "%s", "a step kernel's bounded wait ran out; the state is invalid");
         return fail(h, MMSP_GPU_EOVERFLOW, "%s", "a sparse cell's list outgrew its slots (desc.fields); "
                                                   "the state is invalid");

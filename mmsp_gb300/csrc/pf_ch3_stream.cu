@@ -266,9 +266,10 @@ static F32Coef f32coef(const Coeffs& c)
     return q;
 }
 
-// MMSP_GPU_TEST_STALL_LAUNCHES=n: the next n launches of this kernel in the
-// process run its STALL form, and grids with rows of 64 cells take this
-// kernel too (the failure-detection test).  Read once; unset in normal use.
+// MMSP_GPU_TEST_STALL_LAUNCHES=n: in the next n launches of this kernel and of
+// the ones with a grid barrier in the process the waits run out, and grids with
+// rows of 64 cells take this kernel too (the failure-detection tests).  Read
+// once; unset in normal use.
 static std::atomic<int> g_stall_left{-1};
 static int stall_left()
 {
@@ -281,7 +282,7 @@ static int stall_left()
     }
     return left;
 }
-static int take_stall()
+int take_stall()
 {
     int cur = stall_left();
     while (cur > 0 && !g_stall_left.compare_exchange_weak(cur, cur - 1)) {

@@ -695,6 +695,7 @@ cudaError_t launch_ch64_steps(const Ch64Steps& p, const mmsp_gpu_desc& d, const 
     q.poly0 = (d.model == MMSP_GPU_CH ? 2.0 : c.neg_r) + c.kappa * q.w2;
     P<double> pp = narrow<double>(c, g.dim);
     C64Tiles tl{p.h, p.w, p.nz};
+    if (take_stall()) base += 1u << 30;   // counts that no block will see
     void* args[] = {(void*)&in, (void*)&other, (void*)&g, (void*)&q, (void*)&pp, (void*)&tl, (void*)&steps, (void*)&count,
                     (void*)&base, (void*)&err};
     return cudaLaunchCooperativeKernel(p.fn, dim3(p.blocks), dim3(kC64StepThreads), args, p.smem, s);

@@ -412,7 +412,8 @@ cudaError_t launch_convex_step(const Geom& g, const Coeffs& c, const void* old, 
                                   : (unit ? cs_pick<1, true>(one) : cs_pick<1, false>(one));
     // the reduction scratch: 4 doubles per block, the barrier's count in its last words
     unsigned* count = reinterpret_cast<unsigned*>(partials + 4 * kReduceBlocks);
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), s);
+    // (from 0x80808080 it does not get to the count that the waits are for)
+    cudaError_t e = cudaMemsetAsync(count, take_stall() ? 0x80 : 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&old, (void*)&nw, (void*)&g, (void*)&a, (void*)&partials, (void*)&L, (void*)&count, (void*)&err,
                     (void*)&max_iter, (void*)&first_checks};

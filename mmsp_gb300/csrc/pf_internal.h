@@ -95,6 +95,9 @@ struct StepPlan {
 cudaError_t plan_ch(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 cudaError_t plan_ac(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
 
+// Is this launch one whose waits a failure-detection test has run out (pf_ch3_stream.cu)?
+int take_stall();
+
 // FP32 3D Cahn-Hilliard on rows of 256 cells, states above L2 (pf_ch3_stream.cu).
 bool ch3_stream_eligible(const mmsp_gpu_desc& d, const Geom& g);
 cudaError_t plan_ch3_stream(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p);
