@@ -39,7 +39,7 @@
 namespace pf {
 
 struct AcColF32 {
-    float wx, wy, wz, w2;   // Laplacian weights, w2 = 2 (wx + wy + wz)
+    float wx, wy, wz, w2;   // Laplacian weights (DIFF: negative), w2 = 2 (wx + wy + wz)
     float kappa, dtm, gamma2, neg_r, u;
 };
 
@@ -81,8 +81,13 @@ template <> struct ColVec<4> {
     }
 };
 
-// The new value of one cell, or of a pair in packed FP32x2 instructions, with
-// the polynomial terms regrouped into fewer multiply-adds.
+// The new value of one cell, or of a pair in packed FP32x2 instructions.
+//
+// SUMS: the Laplacian from the sums sx, sy, sz of the two neighbours along each
+// axis, w (hi + lo) - 2 w c, and the polynomial's terms regrouped into fewer
+// multiply-adds.  DIFF: the reference's expressions in its order, the Laplacian
+// from (hi - 2 c) + lo, whose rounding follows the differences and not the
+// cells' own size.  cols_sums below says which grids take which.
 static __device__ __forceinline__ float cfma(float a, float b, float c) { return fmaf(a, b, c); }
 static __device__ __forceinline__ float cmul(float a, float b) { return a * b; }
 static __device__ __forceinline__ float cadd(float a, float b) { return a + b; }
@@ -93,8 +98,14 @@ template <typename VT> static __device__ __forceinline__ VT cset(float k);
 template <> __device__ __forceinline__ float cset<float>(float k) { return k; }
 template <> __device__ __forceinline__ float2 cset<float2>(float k) { return make_float2(k, k); }
 
+template <typename VT>
+static __device__ __forceinline__ VT diff2(VT c, VT lo, VT hi)
+{
+    return cadd(cfma(cset<VT>(-2.0f), c, hi), lo);
+}
+
 template <int MODEL, typename VT>
-static __device__ __forceinline__ VT col_new(VT c, VT sum, VT sx, VT sy, VT sz, const AcColF32& q)
+static __device__ __forceinline__ VT col_new_sums(VT c, VT sum, VT sx, VT sy, VT sz, const AcColF32& q)
 {
     const VT lap = cfma(cset<VT>(q.wx), sx, cfma(cset<VT>(q.wy), sy, cfma(cset<VT>(q.wz), sz, cmul(cset<VT>(-q.w2), c))));
     const VT c2 = cmul(c, c);
@@ -103,15 +114,39 @@ static __device__ __forceinline__ VT col_new(VT c, VT sum, VT sx, VT sy, VT sz, 
         const VT df = cmul(c, cfma(cset<VT>(q.gamma2), sum, cfma(cset<VT>(1.0f - q.gamma2), c2, cset<VT>(-1.0f))));
         return cfma(cset<VT>(-q.dtm), cfma(cset<VT>(-q.kappa), lap, df), c);
     } else if (MODEL == MMSP_GPU_GG || MODEL == MMSP_GPU_ZENER) {
-        // c' = c - dt L (2 (c sum - lap) - c (c^2 + 1))
+        // c' = c - dt L (2 (c sum - lap) - c (c^2 + 1)): the change first, rounded once at the cell's size
         const VT t = cfma(c, sum, cmul(lap, cset<VT>(-1.0f)));
-        const VT m = cmul(c, cadd(c2, cset<VT>(1.0f)));
-        return cfma(cset<VT>(q.dtm), m, cfma(cset<VT>(-2.0f * q.dtm), t, c));
+        const VT m = cmul(c, cfma(cset<VT>(-1.0f), c2, cset<VT>(-1.0f)));
+        return cfma(cset<VT>(-q.dtm), cfma(cset<VT>(2.0f), t, m), c);
     } else {
         // c' = c - dt L (c (u c^2 - r) - kappa lap)
         const VT e = cfma(cset<VT>(-q.kappa), lap, cmul(c, cfma(cset<VT>(q.u), c2, cset<VT>(q.neg_r))));
         return cfma(cset<VT>(-q.dtm), e, c);
     }
+}
+
+// dx, dy, dz: diff2 along each axis.  The Laplacian and the centre enter with
+// the sign that saves a negation.
+template <int MODEL, typename VT>
+static __device__ __forceinline__ VT col_new_diff(VT c, VT sum, VT dx, VT dy, VT dz, const AcColF32& q)
+{
+    const VT neg_lap = cfma(cset<VT>(q.wz), dz, cfma(cset<VT>(q.wy), dy, cmul(cset<VT>(q.wx), dx)));
+    const VT c2 = cmul(c, c);
+    VT e;
+    if (MODEL == MMSP_GPU_AC) {
+        // -c + c^3 + 2 gamma c (sum - c^2) - kappa lap
+        const VT nc = cmul(cset<VT>(-1.0f), c);
+        e = cfma(cmul(cset<VT>(q.gamma2), c), cfma(nc, c, sum), cfma(c2, c, nc));
+        e = cfma(cset<VT>(q.kappa), neg_lap, e);
+    } else if (MODEL == MMSP_GPU_GG || MODEL == MMSP_GPU_ZENER) {
+        // -(-c - c^3 + 2 (c sum - lap))
+        e = cfma(cset<VT>(-2.0f), cfma(c, sum, neg_lap), cfma(c2, c, c));
+        return cfma(cset<VT>(q.dtm), e, c);
+    } else {
+        // -r c + u c^3 - kappa lap
+        e = cfma(cset<VT>(q.kappa), neg_lap, cfma(cset<VT>(q.u), cmul(c2, c), cmul(cset<VT>(q.neg_r), c)));
+    }
+    return cfma(cset<VT>(-q.dtm), e, c);
 }
 
 // Blocks per SM that the registers are held to: 3 (168 registers) where the
@@ -131,7 +166,7 @@ constexpr int cols_min_blocks()
 // rolled values leave registers for several fields' loads in flight, and only
 // a dozen warps share an SM; the loads of plane x+1 then find L2 instead of
 // waiting for HBM.
-template <int N, int V, int MODEL, bool PRE>
+template <int N, int V, int MODEL, bool DIFF, bool PRE>
 __global__ void __launch_bounds__(kAcColThreads, cols_min_blocks<N, V>())
 ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcColF32 q, int planes, int flip)
 {
@@ -195,16 +230,24 @@ ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcC
             if (MODEL == MMSP_GPU_ZENER && f == 0) {
                 w = cc[f];   // Zener pinning: the particles (field 0) have zero mobility
             } else if constexpr (V == 1) {
-                w.v[0] = col_new<MODEL, float>(cc[f].v[0], sum[0], xl[f].v[0] + xh.v[0], yl.v[0] + yh.v[0], zl + zh, q);
+                const float c = cc[f].v[0], xl0 = xl[f].v[0], xh0 = xh.v[0], yl0 = yl.v[0], yh0 = yh.v[0];
+                w.v[0] = DIFF ? col_new_diff<MODEL, float>(c, sum[0], diff2(c, xl0, xh0), diff2(c, yl0, yh0), diff2(c, zl, zh), q)
+                              : col_new_sums<MODEL, float>(c, sum[0], xl0 + xh0, yl0 + yh0, zl + zh, q);
             } else {
 #pragma unroll
                 for (int k = 0; k < V; k += 2) {
-                    const float2 c2 = make_float2(cc[f].v[k], cc[f].v[k + 1]);
-                    const float2 sx = cadd(make_float2(xl[f].v[k], xl[f].v[k + 1]), make_float2(xh.v[k], xh.v[k + 1]));
-                    const float2 sy = cadd(make_float2(yl.v[k], yl.v[k + 1]), make_float2(yh.v[k], yh.v[k + 1]));
-                    const float2 sz = make_float2((k == 0 ? zl : cc[f].v[k - 1]) + cc[f].v[k + 1],
-                                                  cc[f].v[k] + (k + 2 == V ? zh : cc[f].v[k + 2]));
-                    const float2 nv = col_new<MODEL, float2>(c2, make_float2(sum[k], sum[k + 1]), sx, sy, sz, q);
+                    const float2 c2 = make_float2(cc[f].v[k], cc[f].v[k + 1]), s2 = make_float2(sum[k], sum[k + 1]);
+                    const float2 x0 = make_float2(xl[f].v[k], xl[f].v[k + 1]), x1 = make_float2(xh.v[k], xh.v[k + 1]);
+                    const float2 y0 = make_float2(yl.v[k], yl.v[k + 1]), y1 = make_float2(yh.v[k], yh.v[k + 1]);
+                    const float left = k == 0 ? zl : cc[f].v[k - 1], right = k + 2 == V ? zh : cc[f].v[k + 2];
+                    float2 nv;
+                    if (DIFF) {   // (along Z cell by cell: pairs of left and right neighbours would cost moves)
+                        const float2 dz = make_float2(diff2(c2.x, left, c2.y), diff2(c2.y, c2.x, right));
+                        nv = col_new_diff<MODEL, float2>(c2, s2, diff2(c2, x0, x1), diff2(c2, y0, y1), dz, q);
+                    } else {
+                        nv = col_new_sums<MODEL, float2>(c2, s2, cadd(x0, x1), cadd(y0, y1),
+                                                         make_float2(left + c2.y, c2.x + right), q);
+                    }
                     w.v[k] = nv.x;
                     w.v[k + 1] = nv.y;
                 }
@@ -293,13 +336,13 @@ ac_cols_any(const T* __restrict__ ein, T* __restrict__ eout, Geom g, P<T> pc0, i
 
 namespace {
 
-template <int N, int V, bool PRE>
+template <int N, int V, bool DIFF, bool PRE>
 const void* cols_model(int model)
 {
-    if (model == MMSP_GPU_AC) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_AC, PRE>;
-    if (model == MMSP_GPU_GG) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_GG, PRE>;
-    if (model == MMSP_GPU_ZENER) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_ZENER, PRE>;
-    if (N == 1 && model == MMSP_GPU_AC_POLY) return (const void*)&ac_cols_f32<1, V, MMSP_GPU_AC_POLY, PRE>;
+    if (model == MMSP_GPU_AC) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_AC, DIFF, PRE>;
+    if (model == MMSP_GPU_GG) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_GG, DIFF, PRE>;
+    if (model == MMSP_GPU_ZENER) return (const void*)&ac_cols_f32<N, V, MMSP_GPU_ZENER, DIFF, PRE>;
+    if (N == 1 && model == MMSP_GPU_AC_POLY) return (const void*)&ac_cols_f32<1, V, MMSP_GPU_AC_POLY, DIFF, PRE>;
     return nullptr;
 }
 
@@ -309,12 +352,13 @@ const void* cols_model(int model)
 // where the states exceed L2, 127^3 x 6 35.0 / 25.5, x 8 36.9 / 34.8, but 91^3
 // x 7 (42 MB) 12.4 / 13.1 and 127^3 x 10 43.4 / 45.3.  V = 2 never, 128^3 x 8
 // 24.1 / 26.0, 126^3 x 12 44.2 / 45.2.
-template <int N, int V>
+template <int N, int V, bool DIFF>
 const void* cols_pre(int model, bool big)
 {
-    if constexpr (V == 4) return cols_model<N, V, (N >= 6)>(model);
-    else if constexpr (V == 1 && N >= 5 && N <= 9) return big ? cols_model<N, V, true>(model) : cols_model<N, V, false>(model);
-    else return cols_model<N, V, false>(model);
+    if constexpr (V == 4) return cols_model<N, V, DIFF, (N >= 6)>(model);
+    else if constexpr (V == 1 && N >= 5 && N <= 9)
+        return big ? cols_model<N, V, DIFF, true>(model) : cols_model<N, V, DIFF, false>(model);
+    else return cols_model<N, V, DIFF, false>(model);
 }
 
 // V cells per thread, by the row length and the field count: vectors need
@@ -322,22 +366,35 @@ const void* cols_pre(int model, bool big)
 // the vector's alignment), and V*N rolled values must fit the registers.
 // Measured, us per step: 128^3 x 7: 21.7 (V = 4), 31.9 (2), 31.6 (1); x 8:
 // 27.5 / 24.5 / 36.9; x 16: 62 / 55 / 85; 74^3 x 14: 10.3 (V = 2), 12.4 (1).
-template <int V, int LO, int HI>
+template <int V, bool DIFF, int LO, int HI>
 const void* cols_fn(int n, int model, bool big)
 {
     if constexpr (LO > HI) {
         return nullptr;
     } else {
-        return n == LO ? cols_pre<LO, V>(model, big) : cols_fn<V, LO + 1, HI>(n, model, big);
+        return n == LO ? cols_pre<LO, V, DIFF>(model, big) : cols_fn<V, DIFF, LO + 1, HI>(n, model, big);
     }
 }
 
+template <bool DIFF>
 const void* cols_pick(int Z, int n, int model, bool big, int* v)
 {
     *v = Z % 4 == 0 && n <= 7 ? 4 : Z % 2 == 0 && n <= 16 ? 2 : 1;
-    return *v == 4   ? cols_fn<4, 1, 7>(n, model, big)
-           : *v == 2 ? cols_fn<2, 1, 16>(n, model, big)
-                     : cols_fn<1, 1, 32>(n, model, big);
+    return *v == 4   ? cols_fn<4, DIFF, 1, 7>(n, model, big)
+           : *v == 2 ? cols_fn<2, DIFF, 1, 16>(n, model, big)
+                     : cols_fn<1, DIFF, 1, 32>(n, model, big);
+}
+
+// Sums of neighbours on 3D grids of rows of up to 256 cells, unless a plane is
+// one or two rows or a row of all fields more than 5600 values; differences on
+// all others.  Sums are faster where the registers are full, differences round
+// less.  us per step and RMS error against 64 bits after 40 steps, sums /
+// differences: 128^3 x 8 25.0, 1.08e-8 / 29.0, 0.86e-8; 40x50x1000 x 8 27.0,
+// 1.08e-8 / 31.1, 0.84e-8; 30x40x300 x 4 4.1, 1.56e-8 / 4.1, 1.21e-8; 1024^2 x
+// 16 32.9, 0.79e-8 / 32.9, 0.73e-8.
+bool cols_sums(const Geom& g, int n)
+{
+    return g.dim == 3 && g.Z <= 256 && g.Y >= 3 && (long long)g.Z * n <= 5600;
 }
 
 template <typename T, int DIM, bool UNIT>
@@ -397,7 +454,8 @@ cudaError_t plan_ac(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
     }
     const bool big = 2LL * g.cells * d.fields * (long long)sizeof(float) > kAcColL2;
     int v = 1;
-    p->fn = cols_pick(g.Z, d.fields, d.model, big, &v);
+    p->fn = cols_sums(g, d.fields) ? cols_pick<false>(g.Z, d.fields, d.model, big, &v)
+                                   : cols_pick<true>(g.Z, d.fields, d.model, big, &v);
     if (!p->fn) return cudaErrorInvalidConfiguration;
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->fn, kAcColThreads, 0);
@@ -432,10 +490,11 @@ cudaError_t launch_ac(const StepPlan& p, const mmsp_gpu_desc& d, const Geom& g, 
         return cudaLaunchKernel(p.fn, p.grid, p.block, args, p.smem, s);
     }
     // axes that the grid does not have weigh nothing (their neighbours are the cell itself)
+    const float sign = cols_sums(g, n) ? 1.0f : -1.0f;
     AcColF32 q;
-    q.wx = g.dim == 3 ? w.wx : 0.0f;
-    q.wy = g.dim >= 2 ? w.wy : 0.0f;
-    q.wz = w.wz;
+    q.wx = g.dim == 3 ? sign * w.wx : 0.0f;
+    q.wy = g.dim >= 2 ? sign * w.wy : 0.0f;
+    q.wz = sign * w.wz;
     q.w2 = 2.0f * (q.wx + q.wy + q.wz);
     q.kappa = w.kappa;
     q.dtm = w.dtm;
