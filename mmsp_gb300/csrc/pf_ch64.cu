@@ -41,8 +41,9 @@ constexpr int kC64Y = 4;         // rows per block: 128 threads
 // X planes per block (3D): short runs, so that small grids fill the SMs and
 // no SM is left with a long last block.  us per step at 16 / 2 planes, exact
 // form: 40^3 23.3 / 8.4, 100^3 72.3 / 59.7, 33x200x150 59.1 / 50.4, 256^3
-// 742 / 739 (a run of 1 measured as 2).
-constexpr int kC64Planes = 2;
+// 742 / 739 (a run of 1 measured as 2).  Grids of so many planes that the
+// launch's 65535 blocks along X would not do take longer runs, up to 16 planes.
+constexpr int kC64Planes = 2, kC64MostPlanes = 16;
 
 // Constants of both forms.
 struct C64 {
@@ -485,9 +486,9 @@ chf_update(const float* __restrict__ cin, const float* __restrict__ mu, float* _
 
 bool ch64_eligible(const mmsp_gpu_desc& d, const Geom& g)
 {
-    // grid dimensions y and z of the launch stay within 65535 blocks
+    // grid dimensions y and z of the launch stay within 65535 blocks (z with runs of up to kC64MostPlanes planes)
     const long long by = (g.Y + kC64Y - 1) / kC64Y;
-    const long long bz = g.dim == 3 ? (g.X + kC64Planes - 1) / kC64Planes : 1;
+    const long long bz = g.dim == 3 ? (g.X + kC64MostPlanes - 1) / kC64MostPlanes : 1;
     const bool fp64 = d.dtype == MMSP_GPU_F64 && (d.model == MMSP_GPU_CH || d.model == MMSP_GPU_CH_POLY);
     const bool noisy32 = d.dtype == MMSP_GPU_F32 && d.model == MMSP_GPU_CH_POLY && g.dim == 3 && noisy(d);
     return (fp64 || noisy32) && (g.dim == 2 || g.dim == 3) && by <= 65535 && bz <= 65535;
@@ -584,6 +585,7 @@ cudaError_t plan_ch64(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
         warps_y = 1;
         rows = kC64Rows;
     }
+    p->planes = std::max(p->planes, (g.X + 65534) / 65535);
     p->block = dim3(kC64Z, warps_y, 1);
     const int segs = (g.X + p->planes - 1) / p->planes;
     p->grid = dim3((g.Z + kC64Z - 1) / kC64Z, (g.Y + warps_y * rows - 1) / (warps_y * rows), segs);
