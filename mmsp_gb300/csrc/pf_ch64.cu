@@ -44,6 +44,13 @@ constexpr int kC64Y = 4;         // rows per block: 128 threads
 // 742 / 739 (a run of 1 measured as 2).  Grids of so many planes that the
 // launch's 65535 blocks along X would not do take longer runs, up to 16 planes.
 constexpr int kC64Planes = 2, kC64MostPlanes = 16;
+// The stochastic FP32 kernels (below) are bound by the deviates' arithmetic and
+// by HBM, not by the FP64 pipe: short runs, which read more planes twice, are
+// for grids that would leave SMs idle.  us per step at 2 / 8 / 16 planes: 40^3
+// 5.9 / 9.5 / 14.7, 80^3 11.0 / 11.1 / 15.9, 100^3 17.3 / 16.4 / 19.0, 128^3
+// 25.4 / 23.3 / 25.4, 187^3 70.7 / 59.0 / 58.9, 256^3 179 / 146 / 147.
+constexpr int kC32Planes = 8;
+constexpr long long kC32Long = 1000000;   // cells from which on the runs are that long
 
 // Constants of both forms.
 struct C64 {
@@ -570,7 +577,7 @@ cudaError_t plan_ch64(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
                            : mu_fn_m<2>(d.model, c.unit_w, kone, exact, noise);
         p->fn2 = g.dim == 3 ? upd_fn<3>(c.unit_w, exact) : upd_fn<2>(c.unit_w, exact);
     }
-    p->planes = g.dim == 3 ? kC64Planes : 1;
+    p->planes = g.dim != 3 ? 1 : d.dtype == MMSP_GPU_F32 && g.cells >= kC32Long ? kC32Planes : kC64Planes;
     unsigned warps_y = kC64Y, rows = 1;
     // Fewer additions a cell, but threads with more to do: 256^3 412 -> 395 us
     // per step, 224^3 278 -> 269, 187^3 168 -> 164, 160^3 104.5 -> 102.8; but 128^3 55 -> 58.
