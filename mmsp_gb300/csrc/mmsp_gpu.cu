@@ -883,21 +883,24 @@ extern "C" int mmsp_gpu_step(mmsp_gpu_handle* h, int steps)
     const bool captured = capture != cudaStreamCaptureStatusNone;
     int left = steps;
     // (a replay of a captured many-steps launch would wait for barrier counts of the past)
-    if (h->multi && !captured) {
-        while (left > 0) {
-            const int n = std::min(left, kMultiSteps);
-            e = pf::launch_ch64_steps(h->ch64s, h->d, h->g, h->c, h->buf[h->cur], h->buf[h->cur ^ 1], n, multi_word(h),
-                                      h->multi_base, h->flags, h->stream);
-            if (e != cudaSuccess) return cuda_fail(h, e, "steps");
-            h->multi_base += (unsigned)(n - 1) * (unsigned)h->ch64s.blocks;
-            h->cur ^= n & 1;
-            left -= n;
+    while (left > 0 && h->multi && !captured) {
+        const int n = std::min(left, kMultiSteps);
+        e = pf::launch_ch64_steps(h->ch64s, h->d, h->g, h->c, h->buf[h->cur], h->buf[h->cur ^ 1], n, multi_word(h),
+                                  h->multi_base, h->flags, h->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {   // a stream with a part of the SMs: the two passes
+            cudaGetLastError();
+            break;
         }
-    } else if (h->d.model == MMSP_GPU_CH_CONVEX) {
+        if (e != cudaSuccess) return cuda_fail(h, e, "steps");
+        h->multi_base += (unsigned)(n - 1) * (unsigned)h->ch64s.blocks;
+        h->cur ^= n & 1;
+        left -= n;
+    }
+    if (left > 0 && h->d.model == MMSP_GPU_CH_CONVEX) {
         int rc = convex_steps(h, steps);
         if (rc) return rc;
         left = 0;
-    } else {
+    } else if (left > 0) {
         const int launches = h->tb ? left / pf::kTbAnyDepth : left;
         const int rc = captured ? run_captured(h, launches) : run_launches(h, launches);
         if (rc) return rc;

@@ -405,11 +405,13 @@ cudaError_t launch_convex_step(const Geom& g, const Coeffs& c, const void* old, 
     const long long per_color = g.cells / 2, sms = std::min(sm_count(), kReduceBlocks);
     const long long share = (per_color + sms - 1) / sms, rounds = (share + kCsThreads - 1) / kCsThreads;
     const int threads = (int)(((share + rounds - 1) / rounds + 31) / 32 * 32);
-    const int blocks = (int)std::min(sms, (per_color + threads - 1) / threads);
-    const bool one = rounds == 1;
-    const void* fn = g.dim == 3 ? (unit ? cs_pick<3, true>(one) : cs_pick<3, false>(one))
-                     : g.dim == 2 ? (unit ? cs_pick<2, true>(one) : cs_pick<2, false>(one))
-                                  : (unit ? cs_pick<1, true>(one) : cs_pick<1, false>(one));
+    int blocks = (int)std::min(sms, (per_color + threads - 1) / threads);
+    auto pick = [&](bool one) {
+        return g.dim == 3   ? (unit ? cs_pick<3, true>(one) : cs_pick<3, false>(one))
+               : g.dim == 2 ? (unit ? cs_pick<2, true>(one) : cs_pick<2, false>(one))
+                            : (unit ? cs_pick<1, true>(one) : cs_pick<1, false>(one));
+    };
+    const void* fn = pick(rounds == 1);
     // the reduction scratch: 4 doubles per block, the barrier's count in its last words
     unsigned* count = reinterpret_cast<unsigned*>(partials + 4 * kReduceBlocks);
     // (from 0x80808080 it does not get to the count that the waits are for)
@@ -417,7 +419,14 @@ cudaError_t launch_convex_step(const Geom& g, const Coeffs& c, const void* old, 
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&old, (void*)&nw, (void*)&g, (void*)&a, (void*)&partials, (void*)&L, (void*)&count, (void*)&err,
                     (void*)&max_iter, (void*)&first_checks};
-    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, 0, s);
+    e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, 0, s);
+    // a stream with a part of the SMs: fewer blocks, each of which then takes more cells
+    while (e == cudaErrorCooperativeLaunchTooLarge && blocks > 1) {
+        cudaGetLastError();
+        blocks = (blocks + 1) / 2;
+        e = cudaLaunchCooperativeKernel(pick(false), dim3(blocks), dim3(threads), args, 0, s);
+    }
+    return e;
 }
 
 }  // namespace pf
