@@ -371,7 +371,7 @@ static cudaError_t take_kit(size_t bytes, Kit* kit)
     return e;
 }
 
-// `idle`: nothing that uses the set is queued or running.
+// `idle`: nothing that uses the set is queued or running, on any stream.
 static void give_kit(Kit kit, bool idle)
 {
     if (idle && kit.ctx && kit.ctx == context_id() && kit.bytes <= kKitBytes) {
@@ -608,7 +608,9 @@ extern "C" int mmsp_gpu_create(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc)
 extern "C" int mmsp_gpu_destroy(mmsp_gpu_handle* h)
 {
     if (!h) return MMSP_GPU_OK;
-    const bool idle = cudaStreamSynchronize(h->stream) == cudaSuccess;
+    // work of the program's own may still read a state whose address it has asked for, on any stream: its
+    // block goes back to the device, which waits for that, and not to the next handle
+    const bool idle = cudaStreamSynchronize(h->stream) == cudaSuccess && !h->exposed;
     release(h, idle);
     delete h;
     return MMSP_GPU_OK;
@@ -985,6 +987,7 @@ extern "C" int mmsp_gpu_state(mmsp_gpu_handle* h, void** p)
 {
     if (!h || !p) return MMSP_GPU_EINVAL;
     *p = h->buf[h->cur];
+    h->exposed = true;
     return MMSP_GPU_OK;
 }
 

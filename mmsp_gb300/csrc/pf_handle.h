@@ -43,6 +43,7 @@ struct mmsp_gpu_handle {
     unsigned long long kit_ctx;   // the set that own, ev0, ev1 and the block belong to (mmsp_gpu.cu)
     size_t kit_bytes;
     bool timed;              // ev0/ev1 bracket the last step call
+    bool exposed;            // the program has had the address of the state (mmsp_gpu_state)
     bool external;           // buffers and stream belong to the caller (pf::create_in): not freed here
     int64_t steps;
     // CUDA graphs of a short and a long run of launches from buf[0] (at an even launch count of the
