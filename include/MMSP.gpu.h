@@ -190,7 +190,12 @@ int mmsp_gpu_footprint(const mmsp_gpu_desc* desc, size_t* bytes);
  * and a private non-blocking stream. */
 int mmsp_gpu_create(mmsp_gpu_handle** out, const mmsp_gpu_desc* desc);
 
-/* Free the handle's device memory and stream. NULL is accepted. */
+/* Give the handle's device memory and stream back, once its work is done.  Up
+ * to 8 blocks of at most 8 MB each (64 MB) stay with the library, with their
+ * stream, for the next handles that are created; they go back to the device when
+ * an allocation of the library's fails or a server starts.  Larger ones, and any
+ * whose state's address mmsp_gpu_state has given out, are freed here.  NULL is
+ * accepted. */
 int mmsp_gpu_destroy(mmsp_gpu_handle* h);
 
 /* Order the handle's work on an external cudaStream_t (NULL: back to the

@@ -277,8 +277,8 @@ extern "C" int mmsp_gpu_footprint(const mmsp_gpu_desc* d, size_t* bytes)
 // their cudaFrees, which map and unmap memory.  update() of 64 x 64 FP64 cells
 // by 20 steps, host to host: 306 us before, 121 with the sets.
 // At most kKits sets of at most kKitBytes each are held (64 MB), the one given
-// back longest ago going first, and all of them are freed when an allocation
-// fails; larger blocks are freed with their handle.  A set goes to handles of
+// back longest ago going first, and all of them are freed when an allocation of
+// the library fails (pf::device_alloc); larger blocks are freed with their handle.  A set goes to handles of
 // the CUDA context that made it only: its identifier is never used again, so a
 // set that a device reset took away is dropped unread.
 struct Kit {
@@ -288,9 +288,11 @@ struct Kit {
     cudaStream_t stream;
     cudaEvent_t ev0, ev1;
 };
-static const size_t kKits = 8, kKitBytes = 8u << 20;
+static const int kKits = 8;
+static const size_t kKitBytes = 8u << 20;
 static std::mutex g_kits_mu;
-static std::vector<Kit> g_kits;
+static Kit g_kits[kKits];   // the first g_nkits, the longest held first
+static int g_nkits;
 
 static unsigned long long context_id()
 {
@@ -317,51 +319,51 @@ static void free_kit(const Kit& k)
     if (k.stream) cudaStreamDestroy(k.stream);
 }
 
-// The held sets of context `ctx` (0: none), out of the list.
-static std::vector<Kit> drain_kits(unsigned long long ctx)
+// Set i out of the list (under g_kits_mu).
+static Kit remove_kit(int i)
 {
-    std::vector<Kit> mine;
+    const Kit k = g_kits[i];
+    for (g_nkits--; i < g_nkits; i++) g_kits[i] = g_kits[i + 1];
+    return k;
+}
+
+// The smallest held set of context `ctx` with a block of `bytes` and more.
+static bool held_kit(unsigned long long ctx, size_t bytes, Kit* kit)
+{
     std::lock_guard<std::mutex> lock(g_kits_mu);
-    for (size_t i = 0; ctx && i < g_kits.size();) {
-        if (g_kits[i].ctx != ctx) {
-            i++;
-            continue;
-        }
-        mine.push_back(g_kits[i]);
-        g_kits.erase(g_kits.begin() + i);
-    }
-    return mine;
+    int best = -1;
+    for (int i = 0; ctx && i < g_nkits; i++)
+        if (g_kits[i].ctx == ctx && g_kits[i].bytes >= bytes && (best < 0 || g_kits[i].bytes < g_kits[best].bytes))
+            best = i;
+    if (best < 0) return false;
+    *kit = remove_kit(best);
+    return true;
+}
+
+bool pf::free_held_blocks()
+{
+    Kit k;
+    bool any = false;
+    for (const unsigned long long ctx = context_id(); held_kit(ctx, 0, &k); any = true) free_kit(k);
+    return any;
+}
+
+cudaError_t pf::device_alloc(void** p, size_t bytes)
+{
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !free_held_blocks()) return e;
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
 }
 
 static cudaError_t take_kit(size_t bytes, Kit* kit)
 {
-    const unsigned long long ctx = context_id();
-    if (ctx && bytes <= kKitBytes) {
-        std::lock_guard<std::mutex> lock(g_kits_mu);
-        size_t best = g_kits.size();
-        for (size_t i = 0; i < g_kits.size(); i++)
-            if (g_kits[i].ctx == ctx && g_kits[i].bytes >= bytes &&
-                (best == g_kits.size() || g_kits[i].bytes < g_kits[best].bytes))
-                best = i;
-        if (best < g_kits.size()) {
-            *kit = g_kits[best];
-            g_kits.erase(g_kits.begin() + best);
-            return cudaSuccess;
-        }
-    }
+    if (bytes <= kKitBytes && held_kit(context_id(), bytes, kit)) return cudaSuccess;
     *kit = Kit{0, bytes, nullptr, nullptr, nullptr, nullptr};
     cudaError_t e = cudaStreamCreateWithFlags(&kit->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&kit->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&kit->ev1);
-    if (e == cudaSuccess) e = cudaMalloc(&kit->block, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        const std::vector<Kit> held = drain_kits(context_id());
-        for (const Kit& k : held) free_kit(k);
-        if (!held.empty() && kit->ev1) {
-            cudaGetLastError();
-            e = cudaMalloc(&kit->block, bytes);
-        }
-    }
+    if (e == cudaSuccess) e = pf::device_alloc(&kit->block, bytes);
     if (e == cudaSuccess) {
         kit->ctx = context_id();
         return e;
@@ -376,12 +378,17 @@ static void give_kit(Kit kit, bool idle)
 {
     if (idle && kit.ctx && kit.ctx == context_id() && kit.bytes <= kKitBytes) {
         std::lock_guard<std::mutex> lock(g_kits_mu);
-        g_kits.push_back(kit);
-        if (g_kits.size() <= kKits) return;
-        size_t i = 0;
-        while (g_kits[i].ctx != kit.ctx) i++;   // another context's is not this thread's to free
-        kit = g_kits[i];
-        g_kits.erase(g_kits.begin() + i);
+        int i = 0;
+        while (i < g_nkits && g_kits[i].ctx != kit.ctx) i++;
+        if (g_nkits < kKits) {
+            g_kits[g_nkits++] = kit;
+            return;
+        }
+        if (i < kKits) {   // full: the one held longest goes (another context's is not this thread's to free)
+            const Kit out = remove_kit(i);
+            g_kits[g_nkits++] = kit;
+            kit = out;
+        }
     }
     free_kit(kit);
 }

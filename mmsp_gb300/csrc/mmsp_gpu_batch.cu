@@ -189,11 +189,11 @@ extern "C" int mmsp_gpu_batch_create(mmsp_gpu_batch** out, int count, const mmsp
     }
     b->stream = b->own;
     const size_t pool_bytes = (size_t)off * b->esize;
-    bool ok = cudaMalloc(&b->pool[0], pool_bytes) == cudaSuccess && cudaMalloc(&b->pool[1], pool_bytes) == cudaSuccess &&
-              cudaMalloc((void**)&b->partials, kPartialsBytes) == cudaSuccess &&
-              cudaMalloc((void**)&b->counters, 256) == cudaSuccess;
+    bool ok = device_alloc(&b->pool[0], pool_bytes) == cudaSuccess && device_alloc(&b->pool[1], pool_bytes) == cudaSuccess &&
+              device_alloc((void**)&b->partials, kPartialsBytes) == cudaSuccess &&
+              device_alloc((void**)&b->counters, 256) == cudaSuccess;
     if (ok && b->npersistent > 0)
-        ok = cudaMalloc((void**)&b->d_insts, sizeof(BatchInst) * b->insts.size()) == cudaSuccess;
+        ok = device_alloc((void**)&b->d_insts, sizeof(BatchInst) * b->insts.size()) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         brelease(b);
@@ -362,7 +362,7 @@ static int set_items(mmsp_gpu_batch* b, int rows, int threads)
         if (b->d_items) cudaFree(b->d_items);
         b->d_items = nullptr;
         b->items_cap = 0;
-        if (cudaMalloc((void**)&b->d_items, sizeof(BatchItem) * items.size()) != cudaSuccess) {
+        if (device_alloc((void**)&b->d_items, sizeof(BatchItem) * items.size()) != cudaSuccess) {
             cudaGetLastError();
             return bfail(b, MMSP_GPU_ENOMEM, "work list");
         }
@@ -403,7 +403,7 @@ static int set_list(mmsp_gpu_batch* b, const std::vector<Item>& items, Item** li
         if (*list) cudaFree(*list);
         *list = nullptr;
         *cap = 0;
-        if (cudaMalloc((void**)list, sizeof(Item) * items.size()) != cudaSuccess) {
+        if (device_alloc((void**)list, sizeof(Item) * items.size()) != cudaSuccess) {
             cudaGetLastError();
             return bfail(b, MMSP_GPU_ENOMEM, "tile list");
         }

@@ -295,7 +295,7 @@ static int ensure_output(mmsp_gpu_handle* h, size_t bytes)
     s->wait_idle();
     cudaStreamSynchronize(s->copy);
     s->free_buffers();
-    if ((e = cudaMalloc((void**)&s->staging, bytes)) != cudaSuccess ||
+    if ((e = pf::device_alloc((void**)&s->staging, bytes)) != cudaSuccess ||
         (e = cudaHostAlloc((void**)&s->host[0], bytes, cudaHostAllocDefault)) != cudaSuccess ||
         (e = cudaHostAlloc((void**)&s->host[1], bytes, cudaHostAllocDefault)) != cudaSuccess) {
         s->free_buffers();

@@ -370,6 +370,7 @@ extern "C" int mmsp_gpu_server_start(mmsp_gpu_server** out, const mmsp_gpu_serve
     if (!s) return MMSP_GPU_ENOMEM;
     memset(&s->st, 0, sizeof(s->st));
     cudaGetDevice(&s->device);
+    pf::free_held_blocks();   // the budget is a share of what is free
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
@@ -381,7 +382,7 @@ extern "C" int mmsp_gpu_server_start(mmsp_gpu_server** out, const mmsp_gpu_serve
     // the one device block requests are carved from (a little above the budget:
     // blocks are 256-byte aligned per buffer); halve it until the device grants it
     size_t want = s->budget + s->budget / 64 + (64u << 20);
-    while (want >= (64u << 20) && cudaMalloc((void**)&s->pool.base, want) != cudaSuccess) {
+    while (want >= (64u << 20) && pf::device_alloc((void**)&s->pool.base, want) != cudaSuccess) {
         cudaGetLastError();
         want /= 2;
     }

@@ -73,6 +73,10 @@ int sm_count();                 // SMs of the current device
 // plan would break launches of another plan of the same kernel.
 cudaError_t ensure_smem(const void* fn, size_t bytes);
 Coeffs make_coeffs(const mmsp_gpu_desc& d);
+// Free the blocks held for later handles (mmsp_gpu.cu); false: there were none.
+bool free_held_blocks();
+// cudaMalloc; when that fails for want of memory, once more without those blocks.
+cudaError_t device_alloc(void** p, size_t bytes);
 
 // A prepared launch of one explicit step.
 struct StepPlan {
