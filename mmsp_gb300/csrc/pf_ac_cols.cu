@@ -261,7 +261,7 @@ ac_cols_f32(const float* __restrict__ ein, float* __restrict__ eout, Geom g, AcC
 
 
 // ---------------------------------------------------------------------------
-// The new value of one order parameter as ac_new of pf_device.cuh, with the
+// The new value of one order parameter in the reference's order, with the
 // square p2 = phi*phi at hand.  KAPPA: 1 or 2 when kappa is exactly that
 // (1.0*x is x, 2.0*x is exact), 0 for any other value.
 template <typename T, int MODEL, int KAPPA, bool NOISE>
@@ -437,7 +437,6 @@ cudaError_t plan_ac(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
 {
     p->fields = d.fields;
     p->kind = 0;
-    p->ring = 0;
     p->planes = 0;
     // 32-bit byte offsets within a plane need fewer than 2^30 cells
     if (d.dtype == MMSP_GPU_F64 || noisy(d) || g.YZ >= (1LL << 30)) {

@@ -55,14 +55,11 @@ constexpr long long kC32Long = 1000000;   // cells from which on the runs are th
 // Constants of both forms.
 struct C64 {
     double wx, wy, wz;    // Laplacian weights of padded axes X, Y, Z
-    double kappa, dtm, neg_r, u;
+    double kappa, dtm, u;
     double w2;            // 2 (wx + wy + wz) over the real axes: the centre weight
     double poly0;         // contracted mu: 2 + kappa*w2 (CH) or -r + kappa*w2 (CH_POLY)
     double upd0;          // contracted update: -dt*M*w2
     double four, six;     // contracted CH: set in the kernel
-    double noise;
-    unsigned long long seed;
-    long long step;
 };
 
 // The constants of the expressions in registers (Ar::reg).
@@ -549,14 +546,10 @@ C64 c64_of(const Coeffs& c, int dim)
     q.wz = p.wz;
     q.kappa = c.kappa;
     q.dtm = c.dtm;
-    q.neg_r = c.neg_r;
     q.u = c.u;
     q.w2 = 2.0 * (dim == 3 ? p.wx + p.wy + p.wz : p.wy + p.wz);
     q.poly0 = 0.0;   // set by the launcher per model
     q.upd0 = -c.dtm * q.w2;
-    q.noise = c.noise;
-    q.seed = c.seed;
-    q.step = c.step;
     return q;
 }
 
@@ -599,7 +592,6 @@ cudaError_t plan_ch64(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
     p->smem = 0;
     p->fields = 1;
     p->kind = 6;
-    p->ring = 0;
     p->ok = true;
     return cudaSuccess;
 }

@@ -214,27 +214,13 @@ static __device__ __forceinline__ T ch_mu(const Ar<T>& A, T phi, T lap, const P<
     }
 }
 
-// New value of one order parameter of the Allen-Cahn models.
-template <typename T, int MODEL>
-static __device__ __forceinline__ T ac_new(const Ar<T>& A, T phi, T sum, T lap, const P<T>& p)
+// New value of one order parameter of grain growth:
+//   phi - dt*(-phi - pow(phi,3) + 2.0*(phi*sum - lap))   (graingrowth.cpp:105, zener.cpp:135)
+template <typename T>
+static __device__ __forceinline__ T gg_new(const Ar<T>& A, T phi, T sum, T lap, const P<T>& p)
 {
-    if (MODEL == MMSP_GPU_AC) {
-        // phi - dt*L*(-phi + phi*phi*phi + 2.0*gamma*phi*(sum - phi*phi) - kappa*lap)
-        T p2 = A.mul(phi, phi);
-        T p3 = A.mul(p2, phi);
-        T a = A.add(-phi, p3);
-        T g = A.mul(A.mul(p.gamma2, phi), A.sub(sum, p2));
-        T c = A.sub(A.add(a, g), kappa_times(A, p.kappa, lap));
-        return A.sub(phi, A.mul(p.dtm, c));
-    } else if (MODEL == MMSP_GPU_GG || MODEL == MMSP_GPU_ZENER) {
-        // phi - dt*(-phi - pow(phi,3) + 2.0*(phi*sum - lap))   (graingrowth.cpp:105, zener.cpp:135)
-        T e = A.add(A.sub(-phi, cube(A, phi)), twice(A.sub(A.mul(phi, sum), lap)));
-        return A.sub(phi, A.mul(p.dtm, e));
-    } else {
-        // phi - dt*M*(-r*phi + u*pow(phi,3) - K*lap)   (allen-cahn.cpp:70)
-        T e = A.sub(A.add(A.mul(p.neg_r, phi), A.mul(p.u, cube(A, phi))), kappa_times(A, p.kappa, lap));
-        return A.sub(phi, A.mul(p.dtm, e));
-    }
+    T e = A.add(A.sub(-phi, cube(A, phi)), twice(A.sub(A.mul(phi, sum), lap)));
+    return A.sub(phi, A.mul(p.dtm, e));
 }
 
 // The constants of the expressions in registers (Ar::reg).

@@ -91,7 +91,6 @@ struct StepPlan {
                        // 3: FP32 CH rows of any length, 4: Ostwald ripening (two kernels),
                        // 5: convex splitting, 6: FP64 CH in two passes through a work grid,
                        // 8: FP32 3D Ostwald ripening streaming (one kernel)
-    int ring;          // planes in the shared-memory ring (streaming kernels)
     bool ok;
 };
 

@@ -380,7 +380,6 @@ cudaError_t plan_ost3_stream(const mmsp_gpu_desc& d, const Geom& g, const Coeffs
     p->grid = dim3(strips, segs, 1);
     p->fields = N;
     p->kind = 8;
-    p->ring = 0;
     p->ok = true;
     return cudaSuccess;
 }

@@ -258,7 +258,6 @@ cudaError_t plan_ostwald(const mmsp_gpu_desc& d, const Geom& g, StepPlan* p)
     p->planes = 1;
     p->fields = d.fields;
     p->kind = 4;
-    p->ring = 0;
     p->ok = true;
     return cudaSuccess;
 }

@@ -151,7 +151,7 @@ static __device__ __noinline__ void sparse_cell(SpView in, SpView out, Geom g, S
                 if (!UNIT) t = A.mul(q.w[ra], t);
                 lap = ra == 0 ? plus_zero(t) : A.add(lap, t);
             }
-            const double v = ac_new<double, MMSP_GPU_GG>(A, phi, sum, lap, q.p);
+            const double v = gg_new(A, phi, sum, lap, q.p);
             if (v > q.eps) {
                 int h = 0;
                 while (h < dn && out.idx[h * cells + c] != i) h++;
@@ -328,7 +328,7 @@ sparse_gg_step(SpView in, SpView out, Geom g, SpConst q0, int K, int* __restrict
             if (!UNIT) t = A.mul(A.reg(q0.w[ra]), t);
             lap = ra == 0 ? plus_zero(t) : A.add(lap, t);
         }
-        const double v = ac_new<double, MMSP_GPU_GG>(A, phi, sum, lap, p);
+        const double v = gg_new(A, phi, sum, lap, p);
         if (v > q0.eps) {
             int h = (int)(s_pos[s][tid] >> 42) & 63;
             if (!h) {
