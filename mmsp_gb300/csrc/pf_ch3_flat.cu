@@ -18,11 +18,11 @@
 // (the same values).  Odd rows load and store their pairs as two single cells.
 //
 // mu is computed on R + 2 rows for R: the price of keeping it in registers.
-// 187^3: 12.2 us per step = 4.3 TB/s of algorithmic traffic (in L2), bound by
+// 187^3: 13.0 us per step = 4.0 TB/s of algorithmic traffic (in L2), bound by
 // load latency at 12 warps per SM; staging whole rows in a shared-memory ring
 // with a barrier per plane took 22.6 us (62 instructions per cell against
-// 21).  243^3 42.6 -> 26.5, 242^3 34.3 -> 26.0, 208^3 25.9 -> 13.4, 140^3 12.6
-// -> 6.8, 61^3 4.9 -> 3.8, 40^3 4.9 -> 2.7.
+// 21).  243^3 42.6 -> 28.1, 242^3 34.3 -> 26.5, 208^3 25.9 -> 14.9, 140^3 12.6
+// -> 7.4, 61^3 4.9 -> 4.0, 40^3 4.9 -> 2.7.
 #include <algorithm>
 
 #include "pf_device.cuh"
@@ -44,23 +44,23 @@ static __device__ __forceinline__ float2 p2(float a) { return make_float2(a, a);
 // rows above 512 cells, which had the reference's form when all others had
 // sums: RMS error against 64 bits after 40 steps of dt = 0.01, sums /
 // differences, 45x45x513 2.05e-8 / 1.86e-8 (dt = 0.002: 3.01e-8 / 2.99e-8).
-template <bool UNIT, bool DIFF>
-static __device__ __forceinline__ float2 flat_lap(float2 xl, float2 xh, float2 yl, float2 yh, float left, float2 c, float right,
-                                                  const ChFlat& q)
+template <bool UNIT>
+static __device__ __forceinline__ float2 flat_lap(float2 sx, float2 sy, float2 sz, float2 c, const ChFlat& q)
 {
-    float2 sx, sy, sz;
-    if (DIFF) {
-        sx = __fadd2_rn(__ffma2_rn(p2(-2.0f), c, xh), xl);
-        sy = __fadd2_rn(__ffma2_rn(p2(-2.0f), c, yh), yl);
-        sz = p2(fmaf(-2.0f, c.x, c.y) + left, fmaf(-2.0f, c.y, right) + c.x);
-        if (UNIT) return __fadd2_rn(__fadd2_rn(sx, sy), sz);
-        return __ffma2_rn(p2(q.wz), sz, __ffma2_rn(p2(q.wy), sy, __fmul2_rn(p2(q.wx), sx)));
-    }
-    sx = __fadd2_rn(xl, xh);
-    sy = __fadd2_rn(yl, yh);
-    sz = p2(left + c.y, c.x + right);
     if (UNIT) return __ffma2_rn(p2(-6.0f), c, __fadd2_rn(__fadd2_rn(sx, sy), sz));
     return __ffma2_rn(p2(q.wx), sx, __ffma2_rn(p2(q.wy), sy, __ffma2_rn(p2(q.wz), sz, __fmul2_rn(p2(-q.w2), c))));
+}
+
+static __device__ __forceinline__ float2 diff2(float2 lo, float2 c, float2 hi)
+{
+    return __fadd2_rn(__ffma2_rn(p2(-2.0f), c, hi), lo);
+}
+
+template <bool UNIT>
+static __device__ __forceinline__ float2 flat_lap_diff(float2 dx, float2 dy, float2 dz, const ChFlat& q)
+{
+    if (UNIT) return __fadd2_rn(__fadd2_rn(dx, dy), dz);
+    return __ffma2_rn(p2(q.wz), dz, __ffma2_rn(p2(q.wy), dy, __fmul2_rn(p2(q.wx), dx)));
 }
 
 template <int MODEL, bool DIFF>
@@ -81,9 +81,17 @@ static __device__ __forceinline__ float2 flat_mu(float2 c, float2 lap, const ChF
     return __ffma2_rn(p2(-q.kappa), lap, fp);
 }
 
-// the Z neighbours of a lane's pair: the cells left and right of it
-static __device__ __forceinline__ float zleft(float2 c) { return __shfl_up_sync(0xffffffffu, c.y, 1); }
-static __device__ __forceinline__ float zright(float2 c) { return __shfl_down_sync(0xffffffffu, c.x, 1); }
+// sums, or differences, of the two Z neighbours of a lane's pair
+static __device__ __forceinline__ float2 zsum(float2 c)
+{
+    const float left = __shfl_up_sync(0xffffffffu, c.y, 1), right = __shfl_down_sync(0xffffffffu, c.x, 1);
+    return p2(left + c.y, c.x + right);
+}
+static __device__ __forceinline__ float2 zdiff(float2 c)
+{
+    const float left = __shfl_up_sync(0xffffffffu, c.y, 1), right = __shfl_down_sync(0xffffffffu, c.x, 1);
+    return p2(fmaf(-2.0f, c.x, c.y) + left, fmaf(-2.0f, c.y, right) + c.x);
+}
 
 constexpr int kFlatThreads = 128;
 
@@ -150,7 +158,9 @@ ch3_flat_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, Ch
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const float2 v = m[r + 1];
-            const float2 lap = flat_lap<UNIT, DIFF>(ml[r + 1], mh[r + 1], m[r], m[r + 2], zleft(v), v, zright(v), q);
+            const float2 lap =
+                DIFF ? flat_lap_diff<UNIT>(diff2(ml[r + 1], v, mh[r + 1]), diff2(m[r], v, m[r + 2]), zdiff(v), q)
+                     : flat_lap<UNIT>(__fadd2_rn(ml[r + 1], mh[r + 1]), __fadd2_rn(m[r], m[r + 2]), zsum(v), v, q);
             const float2 o = __ffma2_rn(p2(q.dtm), lap, c[r + 2]);
             char* dst = base + (size_t)r * rb;
             if (ODD) {
@@ -165,7 +175,9 @@ ch3_flat_f32(const float* __restrict__ cin, float* __restrict__ cout, Geom g, Ch
 #pragma unroll
         for (int r = 0; r < R + 2; r++) {
             const float2 v = c[r + 1];
-            const float2 lap = flat_lap<UNIT, DIFF>(cl[r + 1], ch[r + 1], c[r], c[r + 2], zleft(v), v, zright(v), q);
+            const float2 lap =
+                DIFF ? flat_lap_diff<UNIT>(diff2(cl[r + 1], v, ch[r + 1]), diff2(c[r], v, c[r + 2]), zdiff(v), q)
+                     : flat_lap<UNIT>(__fadd2_rn(cl[r + 1], ch[r + 1]), __fadd2_rn(c[r], c[r + 2]), zsum(v), v, q);
             m[r] = flat_mu<MODEL, DIFF>(v, lap, q);
         }
     };
