@@ -154,8 +154,8 @@ typedef struct mmsp_gpu_desc {
                          and spinodal.cpp:95-102 (CH_POLY) add gaussian(0, aux[0]) to mu.  The examples
                          draw it from rand() in cell order; here deviate step*cells + cell of a
                          SplitMix64 / Box-Muller stream, step counting from the last upload.
-                         Noisy grids are stepped without graph replay and are refused by batches
-                         and mmsp_gpu_step_noalloc (EUNSUPPORTED). */
+                         Noisy grids are refused by batches and mmsp_gpu_step_noalloc
+                         (EUNSUPPORTED). */
 } mmsp_gpu_desc;
 
 typedef struct mmsp_gpu_stats {

@@ -12,8 +12,8 @@
 // are in registers), so a cell of a field costs 5 loads, one store and about
 // a dozen arithmetic instructions for V = 1.  Offsets within a plane are
 // 32-bit byte offsets, the same for every field and plane; the plane bases
-// are uniform.  Bound: HBM where the two states exceed L2 (128^3 x 8: 24.6 us
-// per step = 5.5 TB/s; x 16: 55 us), else the L1/L2 latency that the resident
+// are uniform.  Bound: HBM where the two states exceed L2 (128^3 x 8: 24.8 us
+// per step = 5.4 TB/s; x 16: 55 us), else the L1/L2 latency that the resident
 // warps leave uncovered.  Streaming whole rows of all fields through a
 // shared-memory ring, one warp per row, took 32.1 and 75.2 us there (it holds
 // 8 to 16 warps per SM), one thread per cell of a row 28.9 us against 10.3 on
@@ -27,10 +27,10 @@
 // doubling is integer arithmetic, and a gradient coefficient of 1 or 2 costs
 // nothing.  19 operations per cell and field for MMSP_GPU_AC with kappa = 2
 // in the reference's order, every one rounded on its own: bit-identical to
-// the reference.  128^3 x 8: 608 us per step, 19 * 16.8 M / 608 us = 0.524 T
+// the reference.  128^3 x 8: 515 us per step, 19 * 16.8 M / 515 us = 0.62 T
 // operations per second; a tile of shared memory with a halo of 1 on a
 // 4-plane ring, 22 operations, took 1100 us (its warps idle at the barriers
-// of each plane), 40x41x42 x 5 16.9 against 84.8, 32^3 x 16 23.0 against 253.
+// of each plane), 40x41x42 x 5 14.1 against 84.8, 32^3 x 16 21.7 against 253.
 #include <algorithm>
 
 #include "pf_device.cuh"
@@ -287,7 +287,8 @@ static __device__ __forceinline__ T ac_new_p2(const Ar<T>& A, T phi, T p2, T sum
 
 // Threads per block: 128, or 32 on grids of few cells, whose warps then
 // spread evenly over the SMs (one FP64 pipe each): 32^3 x 16 fields 25.4 ->
-// 23.0 us per step, 40x41x42 x 5 16.9 -> 15.9; no difference on large grids.
+// 23.0 us per step, 40x41x42 x 5 16.9 -> 15.9 (before the arithmetic of
+// pf_device.cuh, which takes them to 21.7 and 14.1); no difference on large grids.
 constexpr int kAcAnyThreads = 128;
 constexpr long long kAcAnySmall = 1LL << 17;
 

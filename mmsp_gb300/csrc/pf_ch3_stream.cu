@@ -295,7 +295,8 @@ int take_stall()
 // pf_ch3_flat.cu.  us per step, here / there: 256^3 (128 MB) 24.6 / 28.7,
 // 512x256x256 45.0 / 52.5, 200x256x256 (100 MB) 20.5 / 23.9, 160x256x256 (80
 // MB) 17.2 / 18.2; 128x256x256 (64 MB) 14.9 / 14.2.  Every other row length is
-// faster there.
+// faster there (rows of 512 in a ring that walked X one way only: 64x512x512
+// 33.0 / 31.8, 130x512x512 59.7 / 57.7).
 constexpr long long kStreamL2 = 72LL << 20;
 bool ch3_stream_eligible(const mmsp_gpu_desc& d, const Geom& g)
 {

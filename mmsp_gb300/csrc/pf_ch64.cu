@@ -413,9 +413,9 @@ ch64_steps(double* s0, double* s1, Geom g, C64 q0, P<double> p0, C64Tiles tl, in
 // with noise) takes the same two passes: the noise term costs two SplitMix64
 // draws, a logarithm, a cosine and a square root per cell, and a fused kernel
 // would draw it again on every halo; here each deviate is drawn once, in the
-// mu pass, at 8 B per cell of extra traffic (128^3 x 500 steps: 13.0 ms
+// mu pass, at 8 B per cell of extra traffic (128^3 x 500 steps: 11.5 ms
 // against 15.2 ms for the fused row kernel; in 2D the fused tile kernel
-// stays faster, 7.1 ms against 8.3 ms on 1024^2).  Arithmetic as the FP32 form's:
+// stays faster, 7.1 ms against 8.3 ms on 1024^2, 6.5 ms by now).  Arithmetic as the FP32 form's:
 // mu = c (-r + kappa w2 + u c^2) - kappa S + noise, c' = c + dtM (S_mu - w2 mu).
 struct C32 {
     float wx, wy, wz, kappa, u, dtm, poly0, upd0;

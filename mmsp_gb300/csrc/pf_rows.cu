@@ -1,9 +1,10 @@
 // pf_rows.cu -- FP32 Cahn-Hilliard step for rows of any length.
 //
-// The precision-form kernel for 2D (rows up to 1024 cells) and 3D (up to
-// 512) grids that the bulk-copy streaming kernel does not take (rows that
-// are not 32..512 cells in powers of two, or too few rows).  A block owns R rows of the plane (R = 1 in 2D) over their
-// full length, one thread per cell, and streams along axis 0: each thread
+// The precision-form kernel for what the blocked 2D kernels (pf_batch.cu) and
+// the 3D kernels on warp windows (pf_ch3_flat.cu) leave: the last steps of a 2D
+// call, fewer than a block of four (rows up to 1024 cells), and 3D grids with
+// rows of fewer than 4 cells or one row per plane (rows up to 512).  A block
+// owns R rows of the plane (R = 1 in 2D) over their full length, one thread per cell, and streams along axis 0: each thread
 // keeps its column of c for planes x, x+1, x+2 (and the next plane, loaded
 // one plane ahead) and of mu for x-1, x, x+1 in registers.  The Z
 // neighbours of c(x+1) and of mu(x) are read from two small shared-memory

@@ -181,8 +181,8 @@ static __device__ __noinline__ void sparse_cell(SpView in, SpView out, Geom g, S
 // Bound: the FP64 pipe (about 18 operations per cell and grain, and a warp
 // takes as many rounds as its busiest cell; 55% busy) and load latency.  us per
 // step, walking the lists in global memory for every value / here with a row of
-// cells a warp: 512x512 cells of 160 grains 78.5 / 55.1 (500 steps from one item per cell; 60 steps
-// 55.5 / 41.8), 2048x2048 of 32 grains 201 / 154, 48^3 of 12 grains 100 / 58.
+// cells a warp: 512x512 cells of 160 grains 78.5 / 54.9 (500 steps from one item
+// per cell), 2048x2048 of 32 grains 201 / 157, 48^3 of 12 grains 100 / 55.8.
 // (A dense table of a tile's grains in shared memory, behind a hashed
 // dictionary, took 65, 64, 229 and 82: its set-up costs more than the walks.)
 // 64-thread blocks of at most 64 registers: with 128 threads 60.9, with 72
